@@ -63,6 +63,7 @@ struct KParams {
   long long m, n, k, ldd, n_valid;
   int layout, epilogue;
   int m_tiles, n_tiles, splits, kb_total, kb_per_split;
+  int group_m;         // pair kernel: row tiles that are walked together before the next column tile
   int atomic_out;     // fp32 output accumulated with red.global.add (split-K or accumulate mode)
   unsigned lbo_mn, sbo_mn, kstep_mn;  // MN-major descriptor parameters (bytes)
   int peer_mode;       // 0 none, 1 = A row blocks come from peers, 2 = D row blocks go to peers,
@@ -515,6 +516,7 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap *map, uint32
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read_0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -526,22 +528,17 @@ constexpr int EPI_BUF_BYTES = 4096;  // 32 rows x 128 bytes
 constexpr int EPI_STAGING_BYTES = EPI_WARPS * 2 * EPI_BUF_BYTES;
 
 struct EpilogueStaging {
-  uint32_t buf[2];  // shared-memory addresses of this warp's two staging boxes
-  int next;         // which one the next fill uses
+  uint32_t base;  // shared-memory address of this warp's two staging boxes
+  uint32_t next;  // byte offset of the one the next fill uses
 };
 
 // Claims a staging box: the TMA operation that last read it (two fills ago) must have finished
 // reading shared memory.
-__device__ __forceinline__ uint32_t staging_acquire(EpilogueStaging &st, int lane, bool drain_all = false) {
-  if (lane == 0) {
-    if (drain_all)
-      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-    else
-      bulk_wait_read_1();
-  }
+__device__ __forceinline__ uint32_t staging_acquire(EpilogueStaging &st, int lane) {
+  if (lane == 0) bulk_wait_read_1();
   __syncwarp();
-  const uint32_t b = st.buf[st.next];
-  st.next ^= 1;
+  const uint32_t b = st.base + st.next;
+  st.next ^= EPI_BUF_BYTES;
   return b;
 }
 // 16-byte piece `piece` (0..7) of row `lane` inside a swizzled 32 x 128-byte box.
@@ -564,142 +561,261 @@ __device__ __forceinline__ void staging_release(const CUtensorMap *map, uint32_t
   }
 }
 
-// The 64 bytes of the auxiliary operand (residual / pre-activation) that belong to this thread's
-// row in one 32-column chunk. Loaded one chunk ahead of its use so that the global-memory
-// latency overlaps the TMEM read and the math of the previous chunk.
-struct AuxChunk {
-  uint4 v[4];
+// Packed fp32 pairs: sm_100 issues two fp32 FMAs per lane with one instruction, which halves what the GELU and
+// softmax epilogues spend on issue slots. Same IEEE rounding as the scalar operations.
+struct F2 {
+  unsigned long long v;
 };
-__device__ __forceinline__ AuxChunk load_aux_chunk(const KParams &p, long long row, bool row_ok, long long gcol) {
-  AuxChunk a;
-#pragma unroll
-  for (int g = 0; g < 4; ++g) a.v[g] = make_uint4(0u, 0u, 0u, 0u);
-  if (row_ok && gcol < p.n) {
-    const uint4 *ap = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(p.aux) + row * p.ldd + gcol);
-#pragma unroll
-    for (int g = 0; g < 4; ++g)
-      if (gcol + g * 8 + 8 <= p.n) a.v[g] = __ldg(ap + g);
-  }
-  return a;
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_split(F2 x, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_unpack_bf16(uint32_t u) { return f2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
-__device__ __forceinline__ void epilogue_tile_tma(const KParams &p, const CUtensorMap *map_d, const CUtensorMap *map_d2, int m0,
-                                                  int n0, int n_tile, uint32_t tmem_acc, int q, int half, int lane,
-                                                  EpilogueStaging &st, int store_row_base, AuxChunk aux_next) {
-  // store_row_base: first row of the destination tensor map inside the logical output (non-zero
-  // when the rows are scattered to per-owner buffers)
-  const int row0 = m0 + q * 32;
-  const long long row = row0 + lane;
-  const bool row_ok = row < p.m;
-  const bool rows_in_range = row0 < p.m;
-  float run_max = -INFINITY, run_sum = 0.f;
-  const bool f32_out = p.epilogue == kEpiStoreF32 || p.epilogue == kEpiAccumF32;
-  const bool reduce = f32_out && (p.atomic_out || p.epilogue == kEpiAccumF32);
-  uint32_t box = 0, box2 = 0;
-  const bool uses_aux = p.epilogue == kEpiResidualBf16 || p.epilogue == kEpiDGelu;
-#pragma unroll 1
-  for (int ch = 0; ch < 4; ++ch) {
-    const int col0 = half * 128 + ch * 32;
-    const AuxChunk aux = aux_next;
-    if (uses_aux && ch < 3) aux_next = load_aux_chunk(p, row, row_ok, n0 + col0 + 32);
-    uint32_t v[32];
-    tcgen05_ld_32x32b_x32(tmem_acc + col0 + (static_cast<uint32_t>(q * 32) << 16), v);
-    tcgen05_wait_ld();
-    const long long gcol = n0 + col0;
-    const bool cols_in_range = gcol < p.n;
-    float f[32];
+// The same approximation as gelu_math.h (Abramowitz & Stegun 7.1.26), two elements at a time. With
+// u = (1 - erf(|x|/sqrt2)) / 2 = h(t) e,  t = 1 / (1 + 0.3275911 |x|/sqrt2),  e = exp(-x^2/2):
+//   GELU(x)  = max(x, 0) - |x| u            GELU'(x) = 1/2 + copysign(1/2 - u, x) + x e / sqrt(2 pi)
+// h is half the published polynomial. Without the "1 +" of the direct form there is no cancellation for x < 0.
+__device__ __forceinline__ void gelu_tail_pair(F2 ax, F2 x, F2 &h, F2 &e) {
+  float d0, d1, t0, t1, q0, q1;
+  f2_split(f2_fma(ax, f2(0.3275911f * 0.70710678118654752440f, 0.3275911f * 0.70710678118654752440f), f2(1.f, 1.f)), d0, d1);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t0) : "f"(d0));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t1) : "f"(d1));
+  const F2 t = f2(t0, t1);
+  F2 poly = f2_fma(f2(0.5f * 1.061405429f, 0.5f * 1.061405429f), t, f2(0.5f * -1.453152027f, 0.5f * -1.453152027f));
+  poly = f2_fma(poly, t, f2(0.5f * 1.421413741f, 0.5f * 1.421413741f));
+  poly = f2_fma(poly, t, f2(0.5f * -0.284496736f, 0.5f * -0.284496736f));
+  poly = f2_fma(poly, t, f2(0.5f * 0.254829592f, 0.5f * 0.254829592f));
+  h = f2_mul(poly, t);
+  f2_split(f2_mul(f2_mul(x, x), f2(-0.5f * 1.4426950408889634f, -0.5f * 1.4426950408889634f)), q0, q1);
+  e = f2(ex2_approx(q0), ex2_approx(q1));
+}
+// |x| for the tails, where both are zero from 14 on: the bound keeps 0 * inf out of them.
+__device__ __forceinline__ F2 gelu_abs(float a, float b) { return f2(fminf(fabsf(a), 64.f), fminf(fabsf(b), 64.f)); }
+__device__ __forceinline__ uint32_t gelu_pack(float a, float b) {
+  const F2 x = f2(a, b), ax = gelu_abs(a, b);
+  F2 h, e;
+  gelu_tail_pair(ax, x, h, e);
+  float w0, w1, e0, e1;
+  f2_split(f2_mul(ax, h), w0, w1);
+  f2_split(e, e0, e1);
+  return pack_bf16(fmaf(-w0, e0, fmaxf(a, 0.f)), fmaf(-w1, e1, fmaxf(b, 0.f)));
+}
+__device__ __forceinline__ F2 gelu_grad_pair(F2 x) {
+  F2 h, e;
+  float h0, h1, e0, e1, x0, x1;
+  f2_split(x, x0, x1);
+  gelu_tail_pair(gelu_abs(x0, x1), x, h, e);
+  f2_split(h, h0, h1);
+  f2_split(e, e0, e1);
+  const F2 c = f2(0.5f + copysignf(fmaf(-h0, e0, 0.5f), x0), 0.5f + copysignf(fmaf(-h1, e1, 0.5f), x1));
+  return f2_fma(f2_mul(x, f2(0.39894228040143267794f, 0.39894228040143267794f)), e, c);
+}
+
+__device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint32_t (&w)[4]) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
+}
+
+template <int EPI>
+constexpr bool epi_uses_aux = EPI == kEpiResidualBf16 || EPI == kEpiDGelu;
+template <int EPI>
+constexpr bool epi_is_f32 = EPI == kEpiStoreF32;
+// Columns of the tile one epilogue warp handles: half the tile, but never less than one 128-byte box.
+template <int TN, int EPI>
+constexpr int epi_cols = epi_is_f32<EPI> ? TN / 2 : (TN >= 128 ? TN / 2 : 64);
+
+// Auxiliary operand (residual / pre-activation) of one warp's part of a tile: TMA-loaded into the warp's staging boxes,
+// where the result overwrites it. A thread that reads its own row from global memory instead touches 32 rows per load
+// instruction. Called by lane 0, with every earlier store of the warp out of the boxes.
+template <int TN, int EPI>
+__device__ __forceinline__ void aux_prefetch(const CUtensorMap *map_aux, uint32_t box, uint32_t aux_bar, int row0, int col0) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]);
-    if (f32_out) {
-      // one box per 32 fp32 columns
+  for (int g = 0; g < epi_cols<TN, EPI> / 64; ++g) {
+    mbar_expect_tx(aux_bar + 8u * g, EPI_BUF_BYTES);
+    tma_load_2d(box + g * EPI_BUF_BYTES, map_aux, aux_bar + 8u * g, col0 + g * 64, row0);
+  }
+}
+
+// One warp's share of a finished accumulator of the pair kernel: 32 rows of lane quadrant q, epi_cols() columns. What the
+// epilogue does is a template parameter: the softmax and GELU forms are bound by issue slots (13 K cycles a tile with
+// everything decided at run time, against 6 K cycles of tensor-core work for K = 768), and so is what they overlap with.
+// The TMEM load of the next 32 columns is in flight while the current ones are processed, and the accumulator goes back to
+// the MMA warp (`release`) as soon as its last column sits in registers.
+template <int TN, int EPI, typename Release>
+__device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUtensorMap *map_d, const CUtensorMap *map_d2, int m0, int n0,
+                                                   int n_tile, uint32_t tmem_acc, int q, int half, int lane, EpilogueStaging &st,
+                                                   int store_row_base, uint32_t aux_bar, uint32_t aux_parity, volatile int *abort_flag,
+                                                   Release release) {
+  constexpr int COLS = epi_cols<TN, EPI>;
+  constexpr int CHUNKS = COLS / 32;
+  const int row0 = m0 + q * 32;
+  const bool rows_in_range = row0 < p.m;
+  const int col_base = COLS * half;
+  const uint32_t taddr = tmem_acc + col_base + (static_cast<uint32_t>(q * 32) << 16);
+  uint32_t acc[2][32];
+  tcgen05_ld_32x32b_x32(taddr, acc[0]);
+  float run_max = -INFINITY, run_sum = 0.f;  // base-2 softmax partials
+  uint32_t held[EPI == kEpiGeluDual ? 32 : 1];
+  uint32_t box = 0;
+#pragma unroll
+  for (int ch = 0; ch < CHUNKS; ++ch) {
+    uint32_t(&v)[32] = acc[ch & 1];
+    tcgen05_wait_ld();
+    if (ch + 1 < CHUNKS) {
+      tcgen05_ld_32x32b_x32(taddr + (ch + 1) * 32, acc[(ch + 1) & 1]);
+    } else {
+      release();
+    }
+    const int gcol = n0 + col_base + ch * 32;
+    if constexpr (epi_is_f32<EPI>) {
       box = staging_acquire(st, lane);
 #pragma unroll
-      for (int g = 0; g < 8; ++g)
-        st_shared_v4(staging_addr(box, lane, g), v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-      staging_release(map_d, box, static_cast<int>(gcol), row0 - store_row_base, rows_in_range && cols_in_range, reduce, lane);
-      continue;
-    }
-    if (p.bias && cols_in_range) {
-      const uint4 *bp = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(p.bias) + gcol);
+      for (int g = 0; g < 8; ++g) st_shared_v4(staging_addr(box, lane, g), v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+      staging_release(map_d, box, gcol, row0 - store_row_base, rows_in_range && gcol < p.n, p.atomic_out || p.epilogue == kEpiAccumF32, lane);
+    } else {
+      const int sub = ch & 1;  // two 32-column chunks share one 64-column (128-byte) box
+      if (EPI != kEpiDGelu && EPI != kEpiCrossEntropy && p.bias && gcol < p.n) {
+        const uint4 *bp = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(p.bias) + gcol);
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        if (gcol + g * 8 + 8 > p.n) break;
-        const uint4 b = __ldg(bp + g);
-        const uint32_t w[4] = {b.x, b.y, b.z, b.w};
+        for (int g = 0; g < 4; ++g) {
+          if (gcol + g * 8 + 8 > p.n) break;
+          const uint4 b = __ldg(bp + g);
+          const uint32_t w[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 t = unpack_bf16(w[i]);
-          f[g * 8 + 2 * i] += t.x;
-          f[g * 8 + 2 * i + 1] += t.y;
-        }
-      }
-    }
-    if (uses_aux && row_ok && cols_in_range) {
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        if (gcol + g * 8 + 8 > p.n) break;
-        const uint4 a = aux.v[g];
-        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 t = unpack_bf16(w[i]);
-          if (p.epilogue == kEpiResidualBf16) {
-            f[g * 8 + 2 * i] += t.x;
-            f[g * 8 + 2 * i + 1] += t.y;
-          } else {
-            f[g * 8 + 2 * i] *= gelu_grad_f(t.x);
-            f[g * 8 + 2 * i + 1] *= gelu_grad_f(t.y);
+          for (int i = 0; i < 4; ++i) {
+            float s0, s1;
+            f2_split(f2_add(f2(__uint_as_float(v[g * 8 + 2 * i]), __uint_as_float(v[g * 8 + 2 * i + 1])), f2_unpack_bf16(w[i])), s0, s1);
+            v[g * 8 + 2 * i] = __float_as_uint(s0);
+            v[g * 8 + 2 * i + 1] = __float_as_uint(s1);
           }
         }
       }
-    }
-    // two 32-column chunks share one 64-column (128-byte) box
-    const int sub = ch & 1;
-    if (sub == 0) {
-      // the dual-output epilogue fills both boxes at once, so both previous stores must be done
-      box = staging_acquire(st, lane, p.epilogue == kEpiGeluDual);
-      if (p.epilogue == kEpiGeluDual) box2 = staging_acquire(st, lane, true);
-    }
+      if constexpr (epi_uses_aux<EPI>) {
+        if (sub == 0) {
+          box = st.base + (ch >> 1) * EPI_BUF_BYTES;
+          if (!__all_sync(0xffffffffu, mbar_wait(aux_bar + 8u * (ch >> 1), aux_parity, abort_flag))) {
+            tcgen05_wait_ld();  // no load may be outstanding when the kernel unwinds
+            return false;
+          }
+        }
 #pragma unroll
-    for (int g = 0; g < 4; ++g)
-      st_shared_v4(staging_addr(box, lane, sub * 4 + g), pack_bf16(f[g * 8 + 0], f[g * 8 + 1]), pack_bf16(f[g * 8 + 2], f[g * 8 + 3]),
-                   pack_bf16(f[g * 8 + 4], f[g * 8 + 5]), pack_bf16(f[g * 8 + 6], f[g * 8 + 7]));
-    if (p.epilogue == kEpiGeluDual) {
+        for (int g = 0; g < 4; ++g) {
+          uint32_t w[4];
+          ld_shared_v4(staging_addr(box, lane, sub * 4 + g), w);
 #pragma unroll
-      for (int g = 0; g < 4; ++g)
-        st_shared_v4(staging_addr(box2, lane, sub * 4 + g), pack_bf16(gelu_f(f[g * 8 + 0]), gelu_f(f[g * 8 + 1])),
-                     pack_bf16(gelu_f(f[g * 8 + 2]), gelu_f(f[g * 8 + 3])), pack_bf16(gelu_f(f[g * 8 + 4]), gelu_f(f[g * 8 + 5])),
-                     pack_bf16(gelu_f(f[g * 8 + 6]), gelu_f(f[g * 8 + 7])));
-    }
-    if (p.epilogue == kEpiCrossEntropy && row_ok && cols_in_range) {
-      float cmax = -INFINITY;
+          for (int i = 0; i < 4; ++i) {
+            const F2 a = f2_unpack_bf16(w[i]);
+            const F2 x = f2(__uint_as_float(v[g * 8 + 2 * i]), __uint_as_float(v[g * 8 + 2 * i + 1]));
+            float s0, s1;
+            f2_split(EPI == kEpiResidualBf16 ? f2_add(x, a) : f2_mul(x, gelu_grad_pair(a)), s0, s1);
+            w[i] = pack_bf16(s0, s1);
+          }
+          st_shared_v4(staging_addr(box, lane, sub * 4 + g), w[0], w[1], w[2], w[3]);
+        }
+      } else {
+        if (sub == 0) box = staging_acquire(st, lane);
+        uint32_t packed[16];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        f[i] = bf16_round(f[i]);
-        if (gcol + i < p.n_valid) cmax = fmaxf(cmax, f[i]);
+        for (int i = 0; i < 16; ++i) packed[i] = pack_bf16(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+          st_shared_v4(staging_addr(box, lane, sub * 4 + g), packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]);
+        if constexpr (EPI == kEpiGeluDual) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) held[sub * 16 + i] = gelu_pack(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+        }
+        if constexpr (EPI == kEpiCrossEntropy) {
+          // running (max, sum-exp) over the valid columns, on the logits as stored (bf16)
+          constexpr float kLog2e = 1.4426950408889634f;
+          const long long left = p.n_valid - gcol;  // valid columns of this chunk
+          if (left >= 32) {
+            __nv_bfloat162 mx = *reinterpret_cast<__nv_bfloat162 *>(&packed[0]);
+#pragma unroll
+            for (int i = 1; i < 16; ++i) mx = __hmax2(mx, *reinterpret_cast<__nv_bfloat162 *>(&packed[i]));
+            const float cmax = fmaxf(__low2float(mx), __high2float(mx)) * kLog2e;
+            if (cmax > run_max) {
+              run_sum *= ex2_approx(run_max - cmax);  // first chunk: 0 * exp2(-inf) = 0
+              run_max = cmax;
+            }
+            if (run_max > -INFINITY) {
+            const F2 scale = f2(kLog2e, kLog2e), shift = f2(-run_max, -run_max);
+            F2 s0 = f2(0.f, 0.f), s1 = f2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              float a, b, c, d;
+              f2_split(f2_fma(f2_unpack_bf16(packed[i]), scale, shift), a, b);
+              f2_split(f2_fma(f2_unpack_bf16(packed[i + 1]), scale, shift), c, d);
+              s0 = f2_add(s0, f2(ex2_approx(a), ex2_approx(b)));
+              s1 = f2_add(s1, f2(ex2_approx(c), ex2_approx(d)));
+            }
+            float a, b;
+            f2_split(f2_add(s0, s1), a, b);
+            run_sum += a + b;
+            }
+          } else if (left > 0) {
+            float cmax = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const float x = __uint_as_float(i & 1 ? packed[i >> 1] & 0xffff0000u : packed[i >> 1] << 16) * kLog2e;
+              if (i < left) cmax = fmaxf(cmax, x);
+            }
+            if (cmax > run_max) {
+              run_sum *= ex2_approx(run_max - cmax);
+              run_max = cmax;
+            }
+            if (run_max > -INFINITY)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const float x = __uint_as_float(i & 1 ? packed[i >> 1] & 0xffff0000u : packed[i >> 1] << 16);
+              if (i < left) run_sum += ex2_approx(fmaf(x, kLog2e, -run_max));
+            }
+          }
+        }
       }
-      if (cmax > -INFINITY) {
-        const float new_max = fmaxf(run_max, cmax);
-        float s = 0.f;
+      if (sub == 1) {
+        const int c0 = gcol - 32;
+        const bool in_range = rows_in_range && c0 < p.n;
+        staging_release(map_d, box, c0, row0 - store_row_base, in_range, false, lane);
+        if constexpr (EPI == kEpiGeluDual) {
+          const uint32_t box2 = staging_acquire(st, lane);
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (gcol + i < p.n_valid) s += __expf(f[i] - new_max);
-        run_sum = run_sum * __expf(run_max - new_max) + s;
-        run_max = new_max;
+          for (int g = 0; g < 8; ++g) st_shared_v4(staging_addr(box2, lane, g), held[4 * g], held[4 * g + 1], held[4 * g + 2], held[4 * g + 3]);
+          staging_release(map_d2, box2, c0, row0 - store_row_base, in_range, false, lane);
+        }
       }
-    }
-    if (sub == 1) {
-      const int c0 = n0 + half * 128 + (ch - 1) * 32;
-      const bool in_range = rows_in_range && c0 < p.n;
-      staging_release(map_d, box, c0, row0 - store_row_base, in_range, false, lane);
-      if (p.epilogue == kEpiGeluDual) staging_release(map_d2, box2, c0, row0 - store_row_base, in_range, false, lane);
     }
   }
-  if (p.epilogue == kEpiCrossEntropy && row_ok) {
-    float *stp = p.stats + (row * (2LL * p.n_tiles) + 2LL * n_tile + half) * 2;
-    stp[0] = run_max;
-    stp[1] = run_sum;
+  if constexpr (EPI == kEpiCrossEntropy) {
+    const long long row = row0 + lane;
+    if (row < p.m) {
+      float *stp = p.stats + (row * (2LL * p.n_tiles) + 2LL * n_tile + half) * 2;
+      stp[0] = run_max * 0.69314718055994530942f;  // natural logarithm, as the merging kernels expect
+      stp[1] = run_sum;
+    }
   }
+  return true;
 }
 
 // ===================================================================================
@@ -715,11 +831,19 @@ __device__ __forceinline__ void epilogue_tile_tma(const KParams &p, const CUtens
 //   tmem_full[b]  in each CTA (multicast commit); tmem_empty[b] in the leader, counted by the
 //                 epilogue warps of both CTAs
 // ===================================================================================
-constexpr int STAGES2 = 5;
-constexpr int B2_BYTES = 128 * BK * 2;               // this CTA's half of the B tile
-constexpr int STAGE2_BYTES = A_BYTES + B2_BYTES;     // 32 KB
-constexpr int SMEM2_BYTES = STAGES2 * STAGE2_BYTES + EPI_STAGING_BYTES + 1024 + 256;
 constexpr int BM2 = 256;
+constexpr int BARS2_BYTES = 512;
+// Per tile width TN (256, 128 or 64 columns): this CTA's half of the B tile, one stage, and as many stages as fit beside the
+// epilogue's 64 KB.
+template <int TN>
+struct Pair {
+  static constexpr int B_BYTES = TN / 2 * BK * 2;
+  static constexpr int STAGE = A_BYTES + B_BYTES;              // 32 / 24 / 20 KB
+  static constexpr int STAGES = TN == 256 ? 5 : (TN == 128 ? 6 : 7);
+  static constexpr int SMEM = STAGES * STAGE + EPI_STAGING_BYTES + 1024 + BARS2_BYTES;
+  static constexpr int TMEM = 2 * TN;                          // two accumulators
+};
+static_assert(Pair<256>::SMEM <= 232448 && Pair<128>::SMEM <= 232448 && Pair<64>::SMEM <= 232448, "227 KB of shared memory per block");
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -759,12 +883,17 @@ __device__ __forceinline__ void tcgen05_mma_pair(uint32_t tmem_d, uint64_t desc_
       : "memory");
 }
 
+template <int TN>
 __device__ __forceinline__ TileCoord tile_coord2(const KParams &p, int tile) {
   const int mn = p.m_tiles * p.n_tiles;
   const int split = tile / mn;
   const int rem = tile - split * mn;
-  int n_tile = rem / p.m_tiles;
-  int m_tile = rem - n_tile * p.m_tiles;
+  // groups of group_m row tiles walk all column tiles together (see the choice of group_m)
+  const int group = rem / (p.group_m * p.n_tiles);
+  const int in_group = rem - group * p.group_m * p.n_tiles;
+  const int group_rows = min(p.group_m, p.m_tiles - group * p.group_m);
+  int n_tile = in_group / group_rows;
+  int m_tile = group * p.group_m + in_group - n_tile * group_rows;
   if (p.peer_mode == 3) {
     // Rows arrive chunk by chunk from every owner at once: walk the row tiles in arrival order (chunk 0 of every
     // owner starting with this rank, then chunk 1, ...) and finish all column tiles of a row tile before the next.
@@ -785,7 +914,7 @@ __device__ __forceinline__ TileCoord tile_coord2(const KParams &p, int tile) {
   }
   TileCoord c;
   c.m0 = m_tile * BM2;
-  c.n0 = n_tile * BN;
+  c.n0 = n_tile * TN;
   c.n_tile = n_tile;
   c.kb_begin = split * p.kb_per_split;
   c.kb_end = min(p.kb_total, c.kb_begin + p.kb_per_split);
@@ -795,10 +924,15 @@ __device__ __forceinline__ TileCoord tile_coord2(const KParams &p, int tile) {
 // 128 registers per thread (no spills): the SM's four register files are filled by warps, and a partition that
 // holds three of this block's ten warps then still has room for two warps of a light kernel (collectives, AdamW),
 // so those really run beside a resident GEMM block instead of waiting for it to retire.
+// map_aux: auxiliary operand in output boxes (epilogues that have one); map_d2: second output (kEpiGeluDual).
+template <int TN, int EPI>
 __global__ void __maxnreg__(128)
 gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
              const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_d2,
              const __grid_constant__ PeerMaps peer_maps, const KParams p) {
+  constexpr int STAGES2 = Pair<TN>::STAGES, STAGE2_BYTES = Pair<TN>::STAGE;
+  constexpr bool kAux = epi_uses_aux<EPI>;
+  const CUtensorMap &map_aux = map_d2;  // an epilogue has an auxiliary operand or a second output, never both
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -809,8 +943,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES2 + s); };
   auto tmem_full_bar = [&](int b) { return bar_base + 8u * (2 * STAGES2 + b); };
   auto tmem_empty_bar = [&](int b) { return bar_base + 8u * (2 * STAGES2 + 2 + b); };
-  volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(bars + 2 * STAGES2 + 4);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * STAGES2 + 5);
+  auto aux_bar = [&](int w) { return bar_base + 8u * (2 * STAGES2 + 4 + 2 * w); };  // two per epilogue warp
+  volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(bars + 2 * STAGES2 + 4 + 2 * EPI_WARPS);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * STAGES2 + 5 + 2 * EPI_WARPS);
+  static_assert((2 * STAGES2 + 6 + 2 * EPI_WARPS) * 8 <= BARS2_BYTES, "barrier area");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -827,8 +963,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tmem_full_bar(b), 1);
-      mbar_init(tmem_empty_bar(b), 2 * EPI_WARPS);
+      mbar_init(tmem_empty_bar(b), 2 * (epi_cols<TN, EPI> == TN ? EPI_WARPS / 2 : EPI_WARPS));  // warps that read it
     }
+    if (kAux)
+      for (int w = 0; w < 2 * EPI_WARPS; ++w) mbar_init(aux_bar(0) + 8u * w, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
@@ -836,7 +974,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t *>(tmem_slot))),
-                 "r"(TMEM_COLS)
+                 "r"(Pair<TN>::TMEM)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
@@ -854,9 +992,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
       bool ok = true;
       int ready_key = -1;
       for (int tile = pair; ok && tile < total_tiles; tile += num_pairs) {
-        const TileCoord c = tile_coord2(p, tile);
+        const TileCoord c = tile_coord2<TN>(p, tile);
         const int m0 = c.m0 + static_cast<int>(cta) * 128;   // this CTA's rows of A / D
-        const int nb0 = c.n0 + static_cast<int>(cta) * 128;  // this CTA's rows of the B tile
+        const int nb0 = c.n0 + static_cast<int>(cta) * (TN / 2);  // this CTA's rows of the B tile
         if (p.peer_mode == 3) {
           // the rows of this tile are written by the all-gather that runs beside this kernel: wait for their chunk
           const int owner = c.m0 / p.rows_per_peer;
@@ -905,7 +1043,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             tma_load_2d_pair(b_dst, &map_b, full_leader, kb * BK, nb0);
           } else {
 #pragma unroll
-            for (int j = 0; j < 2; ++j) tma_load_2d_pair(b_dst + j * 8192, &map_b, full_leader, nb0 + j * 64, kb * BK);
+            for (int j = 0; j < TN / 128; ++j) tma_load_2d_pair(b_dst + j * 8192, &map_b, full_leader, nb0 + j * 64, kb * BK);
           }
           if (++stage == STAGES2) {
             stage = 0;
@@ -920,7 +1058,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
       const uint32_t a_major = p.layout == kNT ? 1u : 0u;
       const uint32_t b_major = p.layout == kTN ? 0u : 1u;
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (a_major << 15) | (b_major << 16) |
-                             (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(BM2 >> 4) << 24);
+                             (static_cast<uint32_t>(TN >> 3) << 17) | (static_cast<uint32_t>(BM2 >> 4) << 24);
       const uint32_t lbo_a = a_major ? p.lbo_mn : 16u, lbo_b = b_major ? p.lbo_mn : 16u;
       const uint32_t sbo_a = a_major ? p.sbo_mn : 1024u, sbo_b = b_major ? p.sbo_mn : 1024u;
       const uint32_t kstep_a = a_major ? p.kstep_mn : static_cast<uint32_t>(UMMA_K * 2);
@@ -931,10 +1069,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int tile = pair; ok && tile < total_tiles; tile += num_pairs) {
-        const TileCoord c = tile_coord2(p, tile);
+        const TileCoord c = tile_coord2<TN>(p, tile);
         if (!mbar_wait(tmem_empty_bar(acc), acc_phase ^ 1u, abort_flag)) break;
         tcgen05_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * TN;
         for (int kb = c.kb_begin; kb < c.kb_end; ++kb) {
           if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
             ok = false;
@@ -970,34 +1108,48 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     int acc = 0;
     uint32_t acc_phase = 0;
     EpilogueStaging st;
-    st.buf[0] = staging_base + (warp - 2) * 2 * EPI_BUF_BYTES;
-    st.buf[1] = st.buf[0] + EPI_BUF_BYTES;
+    st.base = staging_base + (warp - 2) * 2 * EPI_BUF_BYTES;
     st.next = 0;
-    for (int tile = pair; tile < total_tiles; tile += num_pairs) {
-      const TileCoord c = tile_coord2(p, tile);
-      const int m0_cta = c.m0 + static_cast<int>(cta) * 128;
-      // first chunk of the auxiliary operand is requested before waiting for the accumulator
-      AuxChunk aux0{};
-      if (p.epilogue == kEpiResidualBf16 || p.epilogue == kEpiDGelu) {
-        const long long r = m0_cta + q * 32 + lane;
-        aux0 = load_aux_chunk(p, r, r < p.m, c.n0 + half * 128);
+    constexpr int COLS = epi_cols<TN, EPI>;
+    const bool has_part = half * COLS < TN;  // a 64-column tile has work for one half of the warps only
+    uint32_t aux_parity = 0;
+    auto prefetch = [&](int tile) {
+      if (kAux && lane == 0 && tile < total_tiles) {
+        const TileCoord c = tile_coord2<TN>(p, tile);
+        aux_prefetch<TN, EPI>(&map_aux, st.base, aux_bar(warp - 2), c.m0 + static_cast<int>(cta) * 128 + q * 32, c.n0 + half * COLS);
       }
-      if (!mbar_wait(tmem_full_bar(acc), acc_phase, abort_flag)) break;
-      tcgen05_fence_after();
-      if (p.peer_mode == 2) {
-        // reduce-scatter fused into the epilogue: add this tile into its owner's accumulator
-        const int owner = m0_cta / p.rows_per_peer;
-        epilogue_tile_tma(p, &peer_maps.m[owner], &map_d2, m0_cta, c.n0, c.n_tile, tmem_base + acc * BN, q, half, lane, st,
-                          owner * p.rows_per_peer, aux0);
-      } else {
-        epilogue_tile_tma(p, &map_d, &map_d2, m0_cta, c.n0, c.n_tile, tmem_base + acc * BN, q, half, lane, st, 0, aux0);
-      }
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(tmem_empty_bar(acc), 0));
-      if (++acc == 2) {
-        acc = 0;
-        acc_phase ^= 1u;
+    };
+    if (has_part) {
+      if constexpr (kAux) prefetch(pair);
+      for (int tile = pair; tile < total_tiles; tile += num_pairs) {
+        const TileCoord c = tile_coord2<TN>(p, tile);
+        const int m0_cta = c.m0 + static_cast<int>(cta) * 128;
+        if (!mbar_wait(tmem_full_bar(acc), acc_phase, abort_flag)) break;
+        tcgen05_fence_after();
+        auto release = [&] {
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_shared(tmem_empty_bar(acc), 0));
+        };
+        const CUtensorMap *out = &map_d;
+        int store_base = 0;
+        if (p.peer_mode == 2) {  // reduce-scatter fused into the epilogue: this tile goes to the owner of its rows
+          const int owner = m0_cta / p.rows_per_peer;
+          out = &peer_maps.m[owner];
+          store_base = owner * p.rows_per_peer;
+        }
+        if (!epilogue_pair_tile<TN, EPI>(p, out, &map_d2, m0_cta, c.n0, c.n_tile, tmem_base + acc * TN, q, half, lane, st, store_base,
+                                         aux_bar(warp - 2), aux_parity, abort_flag, release))
+          break;
+        if constexpr (kAux) {
+          if (lane == 0) bulk_wait_read_0();  // the boxes are free again: fetch the next tile's operand behind its main loop
+          prefetch(tile + num_pairs);
+          aux_parity ^= 1u;
+        }
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1u;
+        }
       }
     }
     if (lane == 0) bulk_wait_all();  // this warp's stores have left shared memory and are complete
@@ -1015,7 +1167,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   }
   if (warp == 1) {
     tcgen05_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Pair<TN>::TMEM) : "memory");
   }
 }
 
@@ -1092,6 +1244,72 @@ bool get_tensor_map(const void *ptr, uint64_t inner, uint64_t outer, uint64_t st
 
 }  // namespace
 
+namespace {
+// Row tiles walked together (group_m): the pairs in flight then cover a block of group_m x (pairs / group_m) tiles, and a
+// row panel of A is read from memory once per sweep over the columns. A that stays in L2 as a whole (32 MB of 126 MB, the
+// rest is the other operand and the output passing through) is walked column tile by column tile, so that B streams
+// through once; otherwise blocks of eight, which reads the larger operand of every classifier product once instead of
+// once per column tile.
+int choose_group_m(int64_t m, int64_t k, int m_tiles) {
+  return m * k * 2 <= (32LL << 20) ? m_tiles : 8;
+}
+
+template <int TN, int EPI>
+cudaError_t launch_pair(cudaStream_t s, int grid, const CUtensorMap &a, const CUtensorMap &b, const CUtensorMap &d, const CUtensorMap &d2,
+                        const PeerMaps &peers, const KParams &p) {
+  static const cudaError_t attr_set = cudaFuncSetAttribute(gemm2_kernel<TN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, Pair<TN>::SMEM);
+  if (attr_set != cudaSuccess) return attr_set;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = Pair<TN>::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, gemm2_kernel<TN, EPI>, a, b, d, d2, peers, p);
+}
+template <int TN>
+cudaError_t launch_pair_epi(int epi, cudaStream_t s, int grid, const CUtensorMap &a, const CUtensorMap &b, const CUtensorMap &d,
+                            const CUtensorMap &d2, const PeerMaps &peers, const KParams &p) {
+  switch (epi) {
+    case kEpiStoreBf16: return launch_pair<TN, kEpiStoreBf16>(s, grid, a, b, d, d2, peers, p);
+    case kEpiResidualBf16: return launch_pair<TN, kEpiResidualBf16>(s, grid, a, b, d, d2, peers, p);
+    case kEpiGeluDual: return launch_pair<TN, kEpiGeluDual>(s, grid, a, b, d, d2, peers, p);
+    case kEpiDGelu: return launch_pair<TN, kEpiDGelu>(s, grid, a, b, d, d2, peers, p);
+    case kEpiStoreF32:
+    case kEpiAccumF32: return launch_pair<TN, kEpiStoreF32>(s, grid, a, b, d, d2, peers, p);
+    default: break;
+  }
+  if constexpr (TN == 256) return launch_pair<TN, kEpiCrossEntropy>(s, grid, a, b, d, d2, peers, p);
+  return cudaErrorInvalidValue;
+}
+
+// Width of the pair kernel's tile. A k-block of 64 costs a pair 2 TN cycles of tensor core or 256 + TN cycles of operand
+// traffic (64 bytes a cycle and SM, what the 8192^3 product sustains), whichever is more; a narrower tile pays only where
+// the wide ones leave pairs without work.
+int choose_tile_n(const GemmArgs &a, int pairs, bool fixed) {
+  if (fixed) return 256;
+  int best = 256;
+  double best_cost = 0;
+  for (int tn = 256; tn >= 64; tn /= 2) {
+    if (tn == 64 && a.layout != kTN) break;  // an MN-major half tile of 32 columns is no whole swizzle atom
+    const int64_t tiles = ((a.m + BM2 - 1) / BM2) * ((a.n + tn - 1) / tn);
+    const int64_t waves = (tiles + pairs - 1) / pairs;
+    const double cost = static_cast<double>(waves) * (2 * tn > 256 + tn ? 2 * tn : 256 + tn);
+    if (tn == 256 || cost < 0.95 * best_cost) {
+      best = tn;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+}  // namespace
+
 int64_t gemm_ce_stat_tiles(int64_t n) { return 2 * ((n + BN - 1) / BN); }  // one (max, sum) pair per 128-column half tile
 
 int gemm_status(DeviceStatus *out) {
@@ -1123,7 +1341,15 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
   static const bool one_cta_only = std::getenv("CS_GEMM_1CTA") != nullptr;
   const bool pair_kernel = !one_cta_only && a.m > 128;  // a single 128-row tile gains nothing from pairing
   const int tile_m = pair_kernel ? BM2 : BM;
-  const uint32_t b_box_rows = pair_kernel ? 128u : static_cast<uint32_t>(BN);
+  static const int sm_count = [] {
+    int dev = 0, n = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+  }();
+  const bool peers_used = a.peer_count > 1;
+  const int tn = pair_kernel ? choose_tile_n(a, sm_count / 2, peers_used || f32_out || a.epilogue == kEpiCrossEntropy) : BN;
+  const uint32_t b_box_rows = static_cast<uint32_t>(pair_kernel ? tn / 2 : BN);
   PeerMaps peer_maps{};
   int peer_mode = 0;
   int rows_per_peer = 0;
@@ -1175,7 +1401,8 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
       if (!get_tensor_map(a.d, a.n, a.m, a.ldd, 64, 32, &map_d)) return -1;
     }
     map_d2 = map_d;
-    if (a.d2 && !get_tensor_map(a.d2, a.n, a.m, a.ldd, 64, 32, &map_d2)) return -1;
+    if ((a.epilogue == kEpiResidualBf16 || a.epilogue == kEpiDGelu) && !get_tensor_map(a.aux, a.n, a.m, a.ldd, 64, 32, &map_d2)) return -1;
+    if (a.epilogue == kEpiGeluDual && !get_tensor_map(a.d2, a.n, a.m, a.ldd, 64, 32, &map_d2)) return -1;
   }
 
   KParams p{};
@@ -1192,15 +1419,10 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
   p.layout = a.layout;
   p.epilogue = a.epilogue;
   p.m_tiles = static_cast<int>((a.m + tile_m - 1) / tile_m);
-  p.n_tiles = static_cast<int>((a.n + BN - 1) / BN);
+  p.n_tiles = static_cast<int>((a.n + tn - 1) / tn);
+  p.group_m = choose_group_m(a.m, a.k, p.m_tiles);
   p.kb_total = static_cast<int>((a.k + BK - 1) / BK);
   p.splits = 1;
-  static const int sm_count = [] {
-    int dev = 0, n = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n;
-  }();
   if (f32_out) {
     // Weight gradients have few output tiles and a long reduction: split K so that every SM
     // has work; partial sums meet in the fp32 output through vector atomics.
@@ -1259,8 +1481,7 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
   p.status = status_ptr;
 
   static const bool attr_set = [] {
-    return cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) == cudaSuccess &&
-           cudaFuncSetAttribute(gemm2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES) == cudaSuccess;
+    return cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) == cudaSuccess;
   }();
   if (!attr_set) return -1;
   const int total_tiles = p.m_tiles * p.n_tiles * p.splits;
@@ -1268,19 +1489,9 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
     // a GEMM that waits for chunks of an all-gather in flight leaves SMs free for that gather's blocks
     const int pairs = (sm_count - (peer_mode == 3 ? kGatherBesideGemmBlocks : 0)) / 2;
     const int grid = 2 * (total_tiles < pairs ? total_tiles : pairs);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(grid));
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = SMEM2_BYTES;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm2_kernel, map_a, map_b, map_d, map_d2, peer_maps, p);
+    const cudaError_t e = tn == 256   ? launch_pair_epi<256>(a.epilogue, s, grid, map_a, map_b, map_d, map_d2, peer_maps, p)
+                          : tn == 128 ? launch_pair_epi<128>(a.epilogue, s, grid, map_a, map_b, map_d, map_d2, peer_maps, p)
+                                      : launch_pair_epi<64>(a.epilogue, s, grid, map_a, map_b, map_d, map_d2, peer_maps, p);
     if (e != cudaSuccess) return static_cast<int>(e);
     return finish_launch(1);
   }

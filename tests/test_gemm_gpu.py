@@ -127,3 +127,42 @@ def test_tm_input_gradient_layout(M, N, K):
     F.gelu(x).backward(torch.ones_like(x))
     assert rel(d, ref * x.grad) < 5e-3
     assert C.gemm_status()[0] == 0
+
+
+@pytest.mark.parametrize("layout", [TN, 2])
+@pytest.mark.parametrize("M,N,K", [(129, 8, 72), (384, 72, 200), (1536, 768, 768), (1000, 136, 64), (6000, 1288, 72), (2048, 2304, 328)])
+def test_narrow_tiles_with_every_epilogue(M, N, K, layout):
+    """Shapes whose output has too few 256-column tiles for the chip take 128- or 64-column ones: remainders in rows, columns
+    and K, one column tile and many, with each bf16 epilogue. bf16 results: half an ulp, 2^-9 of the value, in the norm."""
+    a, b = operands(M, N, K)
+    bb = b if layout == TN else b.t().contiguous()
+    ref = a.float() @ b.float().t()
+    aux, bias = torch.randn(M, N, device="cuda").to(BF), torch.randn(N, device="cuda").to(BF)
+    guard = torch.full((M + 3, N + 8), 7.0, device="cuda", dtype=BF)
+    d, d2 = guard[:M, :N], torch.empty(M, N + 8, device="cuda", dtype=BF)[:, :N]
+    assert C.gemm_bf16(a, bb, d, layout, STORE, bias=bias) == 0
+    assert rel(d, ref + bias.float()) < 4e-3
+    wide_aux = torch.empty(M, N + 8, device="cuda", dtype=BF)[:, :N].copy_(aux)  # the auxiliary operand has the output's row stride
+    assert C.gemm_bf16(a, bb, d, layout, RESIDUAL, aux=wide_aux, bias=bias) == 0
+    assert rel(d, ref + bias.float() + aux.float()) < 4e-3
+    assert C.gemm_bf16(a, bb, d, layout, DGELU, aux=wide_aux) == 0
+    x = aux.float().requires_grad_(True)
+    F.gelu(x).backward(torch.ones_like(x))
+    assert rel(d, ref * x.grad) < 5e-3
+    assert C.gemm_bf16(a, bb, d, layout, GELU_DUAL, d2=d2, bias=bias) == 0
+    assert rel(d, ref + bias.float()) < 4e-3 and rel(d2, F.gelu(ref + bias.float())) < 4e-3
+    assert (guard[M:] == 7).all() and (guard[:, N:] == 7).all()
+    assert C.gemm_status()[0] == 0
+
+
+def test_gelu_epilogue_limits():
+    """Infinite and very large pre-activations: GELU is x on the right and zero on the left, never NaN."""
+    a = torch.zeros(256, 64, device="cuda", dtype=BF)
+    a[:, 0] = 1
+    b = torch.zeros(256, 64, device="cuda", dtype=BF)
+    b[:5, 0] = torch.tensor([float("inf"), 3e38, -3e38, -20.0, 20.0])
+    d, d2 = torch.empty(256, 256, device="cuda", dtype=BF), torch.empty(256, 256, device="cuda", dtype=BF)
+    b[0, 1:] = 0
+    assert C.gemm_bf16(a, b, d, TN, GELU_DUAL, d2=d2, bias=None) == 0
+    big = b[1, 0].item()
+    assert d2[7, 1].item() == big and d2[7, 2].item() == 0 and d2[7, 3].item() == 0 and d2[7, 4].item() == 20
