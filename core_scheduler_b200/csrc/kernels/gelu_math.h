@@ -1,5 +1,6 @@
 // SPDX-License-Identifier: Apache-2.0
-// GELU in its exact (erf) form, shared by the GEMM epilogues and the stand-alone GELU kernels.
+// GELU in its exact (erf) form for the stand-alone GELU kernels (the GEMM epilogues evaluate the same approximation on
+// packed pairs).
 #pragma once
 
 namespace cs::kernels {
@@ -8,8 +9,7 @@ namespace {
 // Abramowitz & Stegun (absolute error < 1.5e-7, far below bf16 resolution): one reciprocal, one
 // exponential and five FMAs. GELU'(x) needs exp(-x^2/2) as well, which is the exponential the
 // erf of x/sqrt(2) already computed, so the derivative costs two special-function ops per element
-// instead of the ~45 instructions of erff + expf: the dGELU epilogue stays hidden behind a
-// K = 768 main loop.
+// instead of the ~45 instructions of erff + expf.
 struct ErfParts {
   float erf_abs;  // erf(|x| / sqrt(2))
   float e;        // exp(-x^2 / 2)

@@ -6,13 +6,12 @@
 //                        kNT: A [K,M] and B [K,N] row-major (M/N contiguous) weight gradient
 //                        kTM: A [M,K] row-major, B [K,N] row-major           input gradient (dY * W)
 //
-// Structure (one persistent CTA per SM, 320 threads):
-//   warp 0      TMA producer: cp.async.bulk.tensor tiles -> 4-stage shared-memory ring
-//   warp 1      allocates TMEM and issues tcgen05.mma (one elected lane); 128x256 fp32
-//               accumulators, two of them (512 TMEM columns) so the epilogue of tile i overlaps
-//               the main loop of tile i+1
-//   warps 2-9   epilogue: tcgen05.ld the accumulator (each warp owns a 32-row lane quadrant
-//               and a 128-column half), apply the fused op, store to global memory
+// Structure (one persistent CTA per SM, 320 threads; clusters of two CTAs share a 256-row tile):
+//   warp 0      TMA producer: cp.async.bulk.tensor tiles -> shared-memory ring of five to seven stages
+//   warp 1      allocates TMEM and issues tcgen05.mma (leader CTA); two accumulators, so that the epilogue of
+//               tile i overlaps the main loop of tile i+1
+//   warps 2-9   epilogue: tcgen05.ld the accumulator (each warp owns a 32-row lane quadrant and half of the
+//               columns), apply the fused op, TMA-store to global memory
 // Shared-memory tiles use the 128-byte swizzle; the K-major operands of kTN are described to
 // the MMA with SBO = 1024 B (8 rows x 128 B), the MN-major operands of kNT with LBO = 8192 B
 // (next 64-element block) and SBO = 1024 B (next 8 k-rows).
@@ -35,7 +34,6 @@
 
 #include "api.h"
 #include "bounds_check.h"
-#include "gelu_math.h"
 #include "collectives.h"
 
 namespace cs::kernels {
@@ -43,15 +41,10 @@ namespace {
 constexpr int BM = 128;
 constexpr int BN = 256;
 constexpr int BK = 64;
-constexpr int STAGES = 4;
 constexpr int UMMA_K = 16;
 constexpr int A_BYTES = BM * BK * 2;
-constexpr int B_BYTES = BN * BK * 2;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + EPI_WARPS * 32;
-constexpr int TMEM_COLS = 512;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 constexpr long long kWaitBudgetCycles = 4000000000LL;  // ~2 s at 2 GHz
 
 struct KParams {
@@ -91,9 +84,6 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -118,6 +108,24 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
 }
+// The tensor-core and TMA instructions take their operands from uniform registers. In a branch that one lane took on its own
+// (`if (lane == 0)`) the compiler has to move every operand there again for each instruction: 79 cycles an MMA and 220
+// cycles a k-block of TMA loads were measured, more than the tensor core needs for a tile of 128 columns. So a role's whole
+// warp walks its loop in step and elects a lane only around the instructions themselves; waits are voted on, which keeps
+// the control flow uniform when one of them is abandoned.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok));
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -126,17 +134,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 }
 __device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tcgen05_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tcgen05_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void tcgen05_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -167,337 +164,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t *>(&t);
 }
-__device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
-  return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162 *>(&u));
-}
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 struct TileCoord {
   int m0, n0, kb_begin, kb_end, n_tile;
 };
-__device__ __forceinline__ TileCoord tile_coord(const KParams &p, int tile) {
-  const int mn = p.m_tiles * p.n_tiles;
-  const int split = tile / mn;
-  const int rem = tile - split * mn;
-  const int n_tile = rem / p.m_tiles;
-  const int m_tile = rem - n_tile * p.m_tiles;
-  TileCoord c;
-  c.m0 = m_tile * BM;
-  c.n0 = n_tile * BN;
-  c.n_tile = n_tile;
-  c.kb_begin = split * p.kb_per_split;
-  c.kb_end = min(p.kb_total, c.kb_begin + p.kb_per_split);
-  return c;
-}
-
-// One warp's share of a finished accumulator tile: lane quadrant q (rows m0 + 32q .. +32) and
-// column half `half` (128 of the 256 columns). tmem_acc is the TMEM address of the tile.
-__device__ __forceinline__ void epilogue_tile(const KParams &p, int m0, int n0, int n_tile, uint32_t tmem_acc, int q,
-                                              int half, int lane) {
-  const long long row = m0 + q * 32 + lane;
-  const bool row_ok = row < p.m;
-  float run_max = -INFINITY, run_sum = 0.f;
-#pragma unroll 1
-  for (int ch = 0; ch < 4; ++ch) {
-    const int col0 = half * 128 + ch * 32;
-    uint32_t v[32];
-    tcgen05_ld_32x32b_x32(tmem_acc + col0 + (static_cast<uint32_t>(q * 32) << 16), v);
-    tcgen05_wait_ld();
-    const long long gcol = n0 + col0;
-    if (!row_ok || gcol >= p.n) continue;
-    if (!CS_IN_BOUNDS(kKidGemmEpilogue, row * p.ldd + gcol, static_cast<long long>(p.m) * p.ldd)) continue;
-    float f[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]);
-    if (p.epilogue == kEpiStoreF32 || p.epilogue == kEpiAccumF32) {
-      float *dst = static_cast<float *>(p.d) + row * p.ldd + gcol;
-#pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        if (gcol + g * 4 + 4 > p.n) break;
-        if (p.atomic_out) {
-          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + g * 4), "f"(f[4 * g]),
-                       "f"(f[4 * g + 1]), "f"(f[4 * g + 2]), "f"(f[4 * g + 3])
-                       : "memory");
-        } else {
-          float4 o = make_float4(f[4 * g], f[4 * g + 1], f[4 * g + 2], f[4 * g + 3]);
-          if (p.epilogue == kEpiAccumF32) {
-            const float4 old = *reinterpret_cast<const float4 *>(dst + g * 4);
-            o.x += old.x;
-            o.y += old.y;
-            o.z += old.z;
-            o.w += old.w;
-          }
-          *reinterpret_cast<float4 *>(dst + g * 4) = o;
-        }
-      }
-      continue;
-    }
-    if (p.bias) {
-      const uint4 *bp = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(p.bias) + gcol);
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        if (gcol + g * 8 + 8 > p.n) break;
-        const uint4 b = __ldg(bp + g);
-        const uint32_t w[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 t = unpack_bf16(w[i]);
-          f[g * 8 + 2 * i] += t.x;
-          f[g * 8 + 2 * i + 1] += t.y;
-        }
-      }
-    }
-    __nv_bfloat16 *dst = static_cast<__nv_bfloat16 *>(p.d) + row * p.ldd + gcol;
-    if (p.epilogue == kEpiResidualBf16 || p.epilogue == kEpiDGelu) {
-      const uint4 *ap = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(p.aux) + row * p.ldd + gcol);
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        if (gcol + g * 8 + 8 > p.n) break;
-        const uint4 a = *(ap + g);
-        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 t = unpack_bf16(w[i]);
-          if (p.epilogue == kEpiResidualBf16) {
-            f[g * 8 + 2 * i] += t.x;
-            f[g * 8 + 2 * i + 1] += t.y;
-          } else {
-            f[g * 8 + 2 * i] *= gelu_grad_f(t.x);
-            f[g * 8 + 2 * i + 1] *= gelu_grad_f(t.y);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      if (gcol + g * 8 + 8 > p.n) break;
-      uint4 o;
-      o.x = pack_bf16(f[g * 8 + 0], f[g * 8 + 1]);
-      o.y = pack_bf16(f[g * 8 + 2], f[g * 8 + 3]);
-      o.z = pack_bf16(f[g * 8 + 4], f[g * 8 + 5]);
-      o.w = pack_bf16(f[g * 8 + 6], f[g * 8 + 7]);
-      *reinterpret_cast<uint4 *>(dst + g * 8) = o;
-    }
-    if (p.epilogue == kEpiGeluDual) {
-      __nv_bfloat16 *dst2 = static_cast<__nv_bfloat16 *>(p.d2) + row * p.ldd + gcol;
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        if (gcol + g * 8 + 8 > p.n) break;
-        uint4 o;
-        // GELU of the value as stored (bf16-rounded), so that backward sees the same input
-        o.x = pack_bf16(gelu_f(bf16_round(f[g * 8 + 0])), gelu_f(bf16_round(f[g * 8 + 1])));
-        o.y = pack_bf16(gelu_f(bf16_round(f[g * 8 + 2])), gelu_f(bf16_round(f[g * 8 + 3])));
-        o.z = pack_bf16(gelu_f(bf16_round(f[g * 8 + 4])), gelu_f(bf16_round(f[g * 8 + 5])));
-        o.w = pack_bf16(gelu_f(bf16_round(f[g * 8 + 6])), gelu_f(bf16_round(f[g * 8 + 7])));
-        *reinterpret_cast<uint4 *>(dst2 + g * 8) = o;
-      }
-    }
-    if (p.epilogue == kEpiCrossEntropy) {
-      // running (max, sum-exp) over the valid columns, on the bf16-rounded logits
-      float cmax = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        f[i] = bf16_round(f[i]);
-        if (gcol + i < p.n_valid) cmax = fmaxf(cmax, f[i]);
-      }
-      if (cmax > -INFINITY) {
-        const float new_max = fmaxf(run_max, cmax);
-        float s = 0.f;
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (gcol + i < p.n_valid) s += __expf(f[i] - new_max);
-        run_sum = run_sum * __expf(run_max - new_max) + s;
-        run_max = new_max;
-      }
-    }
-  }
-  if (p.epilogue == kEpiCrossEntropy && row_ok) {
-    float *st = p.stats + (row * (2LL * p.n_tiles) + 2LL * n_tile + half) * 2;
-    st[0] = run_max;
-    st[1] = run_sum;
-  }
-}
-
-// ------------------------------------------------------------------------------ kernel ----
-__global__ void __launch_bounds__(THREADS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const KParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  // 1024-byte alignment: the 128-byte swizzle pattern is a function of the absolute address.
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t *smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem_aligned + STAGES * STAGE_BYTES);
-  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
-  // barrier slots: full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2]
-  auto full_bar = [&](int s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
-  auto tmem_full_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + b); };
-  auto tmem_empty_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + 2 + b); };
-  volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(bars + 2 * STAGES + 4);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * STAGES + 5);
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int total_tiles = p.m_tiles * p.n_tiles * p.splits;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(tmem_full_bar(b), 1);
-      mbar_init(tmem_empty_bar(b), EPI_WARPS);
-    }
-    *abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_b)) : "memory");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t *>(tmem_slot))),
-                 "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tcgen05_fence_before();
-  __syncthreads();
-  tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer ----
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-        const TileCoord c = tile_coord(p, tile);
-        for (int kb = c.kb_begin; kb < c.kb_end; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          const uint32_t a_dst = smem_base + stage * STAGE_BYTES;
-          const uint32_t b_dst = a_dst + A_BYTES;
-          mbar_expect_tx(full_bar(stage), STAGE_BYTES);
-          // K-major operands: one box; MN-major operands: 64-element (128-byte) wide boxes of
-          // 64 k-rows, 8 KB each
-          if (p.layout == kNT) {
-#pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_2d(a_dst + j * 8192, &map_a, full_bar(stage), c.m0 + j * 64, kb * BK);
-          } else {
-            tma_load_2d(a_dst, &map_a, full_bar(stage), kb * BK, c.m0);
-          }
-          if (p.layout == kTN) {
-            tma_load_2d(b_dst, &map_b, full_bar(stage), kb * BK, c.n0);
-          } else {
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j) tma_load_2d(b_dst + j * 8192, &map_b, full_bar(stage), c.n0 + j * 64, kb * BK);
-          }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
-        }
-      }
-      if (!ok) {
-        // Abort path: give loads that are still in flight a bounded chance to land before the
-        // shared memory goes away.
-        for (int s = 0; s < STAGES; ++s) {
-          const long long t0 = clock64();
-          while (!mbar_try_wait(full_bar(s), 0) && !mbar_try_wait(full_bar(s), 1) && clock64() - t0 < 2000000LL) {
-          }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    // -------------------------------------------------------------------- MMA issuer ----
-    if (lane == 0) {
-      const uint32_t a_major = p.layout == kNT ? 1u : 0u;
-      const uint32_t b_major = p.layout == kTN ? 0u : 1u;
-      const uint32_t idesc = (1u << 4) /*fp32 accum*/ | (1u << 7) /*A bf16*/ | (1u << 10) /*B bf16*/ | (a_major << 15) |
-                             (b_major << 16) | (static_cast<uint32_t>(BN >> 3) << 17) |
-                             (static_cast<uint32_t>(BM >> 4) << 24);
-      const uint32_t lbo_a = a_major ? p.lbo_mn : 16u, lbo_b = b_major ? p.lbo_mn : 16u;
-      const uint32_t sbo_a = a_major ? p.sbo_mn : 1024u, sbo_b = b_major ? p.sbo_mn : 1024u;
-      const uint32_t kstep_a = a_major ? p.kstep_mn : static_cast<uint32_t>(UMMA_K * 2);
-      const uint32_t kstep_b = b_major ? p.kstep_mn : static_cast<uint32_t>(UMMA_K * 2);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-        const TileCoord c = tile_coord(p, tile);
-        if (!mbar_wait(tmem_empty_bar(acc), acc_phase ^ 1u, abort_flag)) break;
-        tcgen05_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = c.kb_begin; kb < c.kb_end; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tcgen05_fence_after();
-          const uint32_t a_src = smem_base + stage * STAGE_BYTES;
-          const uint32_t b_src = a_src + A_BYTES;
-#pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t da = make_smem_desc(a_src + k * kstep_a, lbo_a, sbo_a);
-            const uint64_t db = make_smem_desc(b_src + k * kstep_b, lbo_b, sbo_b);
-            tcgen05_mma(d_tmem, da, db, idesc, (kb > c.kb_begin || k > 0) ? 1u : 0u);
-          }
-          tcgen05_commit(empty_bar(stage));  // frees the stage once these MMAs retired
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
-        }
-        if (!ok) break;
-        tcgen05_commit(tmem_full_bar(acc));
-        if (++acc == 2) {
-          acc = 0;
-          acc_phase ^= 1u;
-        }
-      }
-    }
-  } else {
-    // ---------------------------------------------------------------------- epilogue ----
-    const int q = warp & 3;                 // TMEM lane quadrant this warp may access
-    const int half = (warp - 2) >> 2;       // which 128 columns of the tile
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-      const TileCoord c = tile_coord(p, tile);
-      if (!mbar_wait(tmem_full_bar(acc), acc_phase, abort_flag)) break;
-      tcgen05_fence_after();
-      epilogue_tile(p, c.m0, c.n0, c.n_tile, tmem_base + acc * BN, q, half, lane);
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(tmem_empty_bar(acc));
-      if (++acc == 2) {
-        acc = 0;
-        acc_phase ^= 1u;
-      }
-    }
-  }
-
-  // ------------------------------------------------------------------------- teardown ----
-  tcgen05_fence_before();
-  __syncthreads();
-  if (threadIdx.x == 0 && *abort_flag) {
-    p.status->code = 1;
-    p.status->kernel_id = 1;
-    p.status->block = blockIdx.x;
-    p.status->detail = p.layout;
-  }
-  if (warp == 1) {
-    tcgen05_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
-  }
-}
-
-
-
 // ----------------------------------------------------- epilogue through shared memory + TMA ----
 // The accumulator rows a thread reads from TMEM are 64-byte pieces of different output rows;
 // storing them directly makes every store instruction touch 32 half-filled sectors. Instead each
@@ -819,11 +489,10 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
 }
 
 // ===================================================================================
-// 2-CTA variant: a thread-block cluster of two CTAs on neighbouring SMs computes one 256x256
-// tile with tcgen05.mma.cta_group::2. CTA r of the pair loads rows [128r, 128r+128) of the A
-// tile and rows [128r, 128r+128) of the B tile (plain TMA loads, no multicast), so every CTA
-// moves 32 KB per 256x256x64 block instead of 48 KB per 128x256x64 block: one third less
-// L2-to-shared-memory traffic per FLOP, which is what bounds the 1-CTA kernel.
+// A thread-block cluster of two CTAs on neighbouring SMs computes one 256 x TN tile with tcgen05.mma.cta_group::2. CTA r of
+// the pair loads rows [128r, 128r+128) of the A tile and its half of the B tile (plain TMA loads, no multicast): 32 KB a CTA
+// for each 256x256x64 block, where a CTA on its own would move 48 KB for 128x256x64. One row tile of up to 128 rows runs
+// with the second CTA's half empty.
 // The leader CTA (cluster rank 0) issues the MMAs for the pair; barriers:
 //   full[s]       in the leader: the leader's producer arrives with the byte count of both
 //                 CTAs, both CTAs' TMA loads complete on it
@@ -948,7 +617,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * STAGES2 + 5 + 2 * EPI_WARPS);
   static_assert((2 * STAGES2 + 6 + 2 * EPI_WARPS) * 8 <= BARS2_BYTES, "barrier area");
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();
   const bool leader = cta == 0;
@@ -982,62 +651,66 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers exist before anyone signals across the pair
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     // ---------------------------------------------- TMA producer (one per CTA) ----
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int ready_key = -1;
-      for (int tile = pair; ok && tile < total_tiles; tile += num_pairs) {
-        const TileCoord c = tile_coord2<TN>(p, tile);
-        const int m0 = c.m0 + static_cast<int>(cta) * 128;   // this CTA's rows of A / D
-        const int nb0 = c.n0 + static_cast<int>(cta) * (TN / 2);  // this CTA's rows of the B tile
-        if (p.peer_mode == 3) {
-          // the rows of this tile are written by the all-gather that runs beside this kernel: wait for their chunk
-          const int owner = c.m0 / p.rows_per_peer;
-          const int chunk = (c.m0 - owner * p.rows_per_peer) / (p.rows_per_peer / p.ready_chunks);
-          const int key = owner * 8 + chunk;
-          if (key != ready_key) {
-            const uint32_t *flag = p.ready_flags + key;
-            const long long t0 = clock64();
-            for (;;) {
-              uint32_t seen;
-              asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
-              if (static_cast<int32_t>(seen - p.ready_epoch) >= 0) break;
-              if (*abort_flag || clock64() - t0 > kWaitBudgetCycles) {
-                *abort_flag = 1;
-                ok = false;
-                break;
-              }
-              __nanosleep(100);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int ready_key = -1;
+    for (int tile = pair; ok && tile < total_tiles; tile += num_pairs) {
+      const TileCoord c = tile_coord2<TN>(p, tile);
+      const int m0 = c.m0 + static_cast<int>(cta) * 128;         // this CTA's rows of A / D
+      const int nb0 = c.n0 + static_cast<int>(cta) * (TN / 2);   // this CTA's rows of the B tile
+      const CUtensorMap *rows_map = &map_a;
+      int row = m0;
+      if (p.peer_mode == 1) {  // all-gather fused into the load: this tile's rows live in their owner's memory
+        const int owner = m0 / p.rows_per_peer;
+        rows_map = &peer_maps.m[owner];
+        row = m0 - owner * p.rows_per_peer;
+      }
+      if (p.peer_mode == 3) {
+        // the rows of this tile are written by the all-gather that runs beside this kernel: wait for their chunk
+        const int owner = c.m0 / p.rows_per_peer;
+        const int chunk = (c.m0 - owner * p.rows_per_peer) / (p.rows_per_peer / p.ready_chunks);
+        const int key = owner * 8 + chunk;
+        if (key != ready_key) {
+          const uint32_t *flag = p.ready_flags + key;
+          const long long t0 = clock64();
+          for (;;) {
+            uint32_t seen;
+            asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
+            if (static_cast<int32_t>(seen - p.ready_epoch) >= 0) break;
+            if (*abort_flag || clock64() - t0 > kWaitBudgetCycles) {
+              *abort_flag = 1;
+              ok = false;
+              break;
             }
-            if (!ok) break;
-            // the chunk was written by other GPUs through the generic proxy; the loads below go through the async proxy
-            asm volatile("fence.proxy.async.global;" ::: "memory");
-            ready_key = key;
+            __nanosleep(100);
           }
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          // the chunk was written by other GPUs through the generic proxy; the loads below go through the async proxy
+          asm volatile("fence.proxy.async.global;" ::: "memory");
+          ready_key = key;
         }
-        for (int kb = c.kb_begin; kb < c.kb_end; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          const uint32_t a_dst = smem_base + stage * STAGE2_BYTES;
-          const uint32_t b_dst = a_dst + A_BYTES;
-          const uint32_t full_leader = mapa_shared(full_bar(stage), 0);
+      }
+      for (int kb = c.kb_begin; kb < c.kb_end; ++kb) {
+        if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        const uint32_t a_dst = smem_base + stage * STAGE2_BYTES;
+        const uint32_t b_dst = a_dst + A_BYTES;
+        const uint32_t full_leader = mapa_shared(full_bar(stage), 0);
+        if (elect_one()) {
           if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE2_BYTES);
           if (p.layout == kNT) {
 #pragma unroll
             for (int j = 0; j < 2; ++j) tma_load_2d_pair(a_dst + j * 8192, &map_a, full_leader, m0 + j * 64, kb * BK);
-          } else if (p.peer_mode == 1) {
-            // all-gather fused into the load: this tile's rows live in their owner's memory
-            const int owner = m0 / p.rows_per_peer;
-            tma_load_2d_pair(a_dst, &peer_maps.m[owner], full_leader, kb * BK, m0 - owner * p.rows_per_peer);
           } else {
-            tma_load_2d_pair(a_dst, &map_a, full_leader, kb * BK, m0);
+            tma_load_2d_pair(a_dst, rows_map, full_leader, kb * BK, row);
           }
           if (p.layout == kTN) {
             tma_load_2d_pair(b_dst, &map_b, full_leader, kb * BK, nb0);
@@ -1045,24 +718,25 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
 #pragma unroll
             for (int j = 0; j < TN / 128; ++j) tma_load_2d_pair(b_dst + j * 8192, &map_b, full_leader, nb0 + j * 64, kb * BK);
           }
-          if (++stage == STAGES2) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        if (++stage == STAGES2) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer (leader CTA only) ----
-    if (lane == 0 && leader) {
+    if (leader) {
       const uint32_t a_major = p.layout == kNT ? 1u : 0u;
       const uint32_t b_major = p.layout == kTN ? 0u : 1u;
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (a_major << 15) | (b_major << 16) |
                              (static_cast<uint32_t>(TN >> 3) << 17) | (static_cast<uint32_t>(BM2 >> 4) << 24);
-      const uint32_t lbo_a = a_major ? p.lbo_mn : 16u, lbo_b = b_major ? p.lbo_mn : 16u;
-      const uint32_t sbo_a = a_major ? p.sbo_mn : 1024u, sbo_b = b_major ? p.sbo_mn : 1024u;
-      const uint32_t kstep_a = a_major ? p.kstep_mn : static_cast<uint32_t>(UMMA_K * 2);
-      const uint32_t kstep_b = b_major ? p.kstep_mn : static_cast<uint32_t>(UMMA_K * 2);
+      // descriptors of stage 0; a stage or a k-step further only moves the 16-byte-unit address field
+      const uint64_t desc_a = make_smem_desc(smem_base, a_major ? p.lbo_mn : 16u, a_major ? p.sbo_mn : 1024u);
+      const uint64_t desc_b = make_smem_desc(smem_base + A_BYTES, b_major ? p.lbo_mn : 16u, b_major ? p.sbo_mn : 1024u);
+      const uint32_t kstep_a = (a_major ? p.kstep_mn : static_cast<uint32_t>(UMMA_K * 2)) >> 4;
+      const uint32_t kstep_b = (b_major ? p.kstep_mn : static_cast<uint32_t>(UMMA_K * 2)) >> 4;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -1070,31 +744,30 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
       bool ok = true;
       for (int tile = pair; ok && tile < total_tiles; tile += num_pairs) {
         const TileCoord c = tile_coord2<TN>(p, tile);
-        if (!mbar_wait(tmem_empty_bar(acc), acc_phase ^ 1u, abort_flag)) break;
+        if (!mbar_wait_warp(tmem_empty_bar(acc), acc_phase ^ 1u, abort_flag)) break;
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TN;
         for (int kb = c.kb_begin; kb < c.kb_end; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
+          if (!mbar_wait_warp(full_bar(stage), phase, abort_flag)) {
             ok = false;
             break;
           }
           tcgen05_fence_after();
-          const uint32_t a_src = smem_base + stage * STAGE2_BYTES;
-          const uint32_t b_src = a_src + A_BYTES;
+          const uint64_t da = desc_a + static_cast<uint32_t>(stage * (STAGE2_BYTES >> 4));
+          const uint64_t db = desc_b + static_cast<uint32_t>(stage * (STAGE2_BYTES >> 4));
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t da = make_smem_desc(a_src + k * kstep_a, lbo_a, sbo_a);
-            const uint64_t db = make_smem_desc(b_src + k * kstep_b, lbo_b, sbo_b);
-            tcgen05_mma_pair(d_tmem, da, db, idesc, (kb > c.kb_begin || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              tcgen05_mma_pair(d_tmem, da + k * kstep_a, db + k * kstep_b, idesc, (kb > c.kb_begin || k > 0) ? 1u : 0u);
+            tcgen05_commit_pair(empty_bar(stage));
+            if (kb + 1 == c.kb_end) tcgen05_commit_pair(tmem_full_bar(acc));
           }
-          tcgen05_commit_pair(empty_bar(stage));
           if (++stage == STAGES2) {
             stage = 0;
             phase ^= 1u;
           }
         }
         if (!ok) break;
-        tcgen05_commit_pair(tmem_full_bar(acc));
         if (++acc == 2) {
           acc = 0;
           acc_phase ^= 1u;
@@ -1152,7 +825,13 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         }
       }
     }
-    if (lane == 0) bulk_wait_all();  // this warp's stores have left shared memory and are complete
+    // the shared memory must outlive the stores that read it; stores into peers are complete before the block ends
+    if (lane == 0) {
+      if (p.peer_mode == 2)
+        bulk_wait_all();
+      else
+        bulk_wait_read_0();
+    }
   }
 
   // ------------------------------------------------------------------------- teardown ----
@@ -1291,7 +970,8 @@ cudaError_t launch_pair_epi(int epi, cudaStream_t s, int grid, const CUtensorMap
 
 // Width of the pair kernel's tile. A k-block of 64 costs a pair 2 TN cycles of tensor core or 256 + TN cycles of operand
 // traffic (64 bytes a cycle and SM, what the 8192^3 product sustains), whichever is more; a narrower tile pays only where
-// the wide ones leave pairs without work.
+// the wide ones leave pairs without work. Measured with 256 / 128 / 64 columns: 1536x768x3072 21.2 / 13.6 / 13.4 us,
+// 1536x2304x768 10.8 / 10.6 / 12.0, 3000x5120x1280 42.0 / 43.5 / 57.2, 16384x768x3072 60.5 / 65.9 / 92.6.
 int choose_tile_n(const GemmArgs &a, int pairs, bool fixed) {
   if (fixed) return 256;
   int best = 256;
@@ -1338,9 +1018,6 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
   static const bool disabled = std::getenv("CS_DISABLE_TCGEN05_GEMM") != nullptr;
   if (disabled) return -1;
 
-  static const bool one_cta_only = std::getenv("CS_GEMM_1CTA") != nullptr;
-  const bool pair_kernel = !one_cta_only && a.m > 128;  // a single 128-row tile gains nothing from pairing
-  const int tile_m = pair_kernel ? BM2 : BM;
   static const int sm_count = [] {
     int dev = 0, n = 148;
     cudaGetDevice(&dev);
@@ -1348,13 +1025,13 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
     return n;
   }();
   const bool peers_used = a.peer_count > 1;
-  const int tn = pair_kernel ? choose_tile_n(a, sm_count / 2, peers_used || f32_out || a.epilogue == kEpiCrossEntropy) : BN;
-  const uint32_t b_box_rows = static_cast<uint32_t>(pair_kernel ? tn / 2 : BN);
+  const int tn = choose_tile_n(a, sm_count / 2, peers_used || f32_out || a.epilogue == kEpiCrossEntropy);
+  const uint32_t b_box_rows = static_cast<uint32_t>(tn / 2);
   PeerMaps peer_maps{};
   int peer_mode = 0;
   int rows_per_peer = 0;
   if (a.peer_count > 1) {
-    if (!pair_kernel || a.peer_count > 8 || a.m % a.peer_count != 0) return -1;
+    if (a.peer_count > 8 || a.m % a.peer_count != 0) return -1;
     rows_per_peer = static_cast<int>(a.m / a.peer_count);
     if (rows_per_peer % BM2 != 0) return -1;
     if (a.a_peers[0]) {
@@ -1391,19 +1068,17 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
     if (!get_tensor_map(a.b, a.n, a.k, a.ldb, 64, BK, &map_b)) return -1;
   }
   CUtensorMap map_d{}, map_d2{};
-  if (pair_kernel) {
-    // output boxes of the TMA-store epilogue: 32 rows x 128 bytes
-    if (peer_mode == 2) {
-      map_d = peer_maps.m[0];
-    } else if (f32_out) {
-      if (!get_tensor_map(a.d, a.n, a.m, a.ldd, 32, 32, &map_d, 4)) return -1;
-    } else {
-      if (!get_tensor_map(a.d, a.n, a.m, a.ldd, 64, 32, &map_d)) return -1;
-    }
-    map_d2 = map_d;
-    if ((a.epilogue == kEpiResidualBf16 || a.epilogue == kEpiDGelu) && !get_tensor_map(a.aux, a.n, a.m, a.ldd, 64, 32, &map_d2)) return -1;
-    if (a.epilogue == kEpiGeluDual && !get_tensor_map(a.d2, a.n, a.m, a.ldd, 64, 32, &map_d2)) return -1;
+  // output boxes of the TMA-store epilogue: 32 rows x 128 bytes
+  if (peer_mode == 2) {
+    map_d = peer_maps.m[0];
+  } else if (f32_out) {
+    if (!get_tensor_map(a.d, a.n, a.m, a.ldd, 32, 32, &map_d, 4)) return -1;
+  } else {
+    if (!get_tensor_map(a.d, a.n, a.m, a.ldd, 64, 32, &map_d)) return -1;
   }
+  map_d2 = map_d;
+  if ((a.epilogue == kEpiResidualBf16 || a.epilogue == kEpiDGelu) && !get_tensor_map(a.aux, a.n, a.m, a.ldd, 64, 32, &map_d2)) return -1;
+  if (a.epilogue == kEpiGeluDual && !get_tensor_map(a.d2, a.n, a.m, a.ldd, 64, 32, &map_d2)) return -1;
 
   KParams p{};
   p.d = a.d;
@@ -1418,7 +1093,7 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
   p.n_valid = a.n_valid > 0 ? a.n_valid : a.n;
   p.layout = a.layout;
   p.epilogue = a.epilogue;
-  p.m_tiles = static_cast<int>((a.m + tile_m - 1) / tile_m);
+  p.m_tiles = static_cast<int>((a.m + BM2 - 1) / BM2);
   p.n_tiles = static_cast<int>((a.n + tn - 1) / tn);
   p.group_m = choose_group_m(a.m, a.k, p.m_tiles);
   p.kb_total = static_cast<int>((a.k + BK - 1) / BK);
@@ -1427,7 +1102,7 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
     // Weight gradients have few output tiles and a long reduction: split K so that every SM
     // has work; partial sums meet in the fp32 output through vector atomics.
     const int mn = p.m_tiles * p.n_tiles;
-    const int workers = pair_kernel ? sm_count / 2 : sm_count;
+    const int workers = sm_count / 2;
     // Pick the split count whose tile total fills whole waves of `workers` best, keeping at
     // least 8 k-blocks per split; ties go to fewer splits (fewer reduce-adds).
     const int max_splits = p.kb_total / 8 > 0 ? p.kb_total / 8 : 1;
@@ -1480,23 +1155,14 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
   }();
   p.status = status_ptr;
 
-  static const bool attr_set = [] {
-    return cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) == cudaSuccess;
-  }();
-  if (!attr_set) return -1;
   const int total_tiles = p.m_tiles * p.n_tiles * p.splits;
-  if (pair_kernel) {
-    // a GEMM that waits for chunks of an all-gather in flight leaves SMs free for that gather's blocks
-    const int pairs = (sm_count - (peer_mode == 3 ? kGatherBesideGemmBlocks : 0)) / 2;
-    const int grid = 2 * (total_tiles < pairs ? total_tiles : pairs);
-    const cudaError_t e = tn == 256   ? launch_pair_epi<256>(a.epilogue, s, grid, map_a, map_b, map_d, map_d2, peer_maps, p)
-                          : tn == 128 ? launch_pair_epi<128>(a.epilogue, s, grid, map_a, map_b, map_d, map_d2, peer_maps, p)
-                                      : launch_pair_epi<64>(a.epilogue, s, grid, map_a, map_b, map_d, map_d2, peer_maps, p);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    return finish_launch(1);
-  }
-  const int grid = total_tiles < sm_count ? total_tiles : sm_count;
-  gemm_kernel<<<grid, THREADS, SMEM_BYTES, s>>>(map_a, map_b, p);
+  // a GEMM that waits for chunks of an all-gather in flight leaves SMs free for that gather's blocks
+  const int pairs = (sm_count - (peer_mode == 3 ? kGatherBesideGemmBlocks : 0)) / 2;
+  const int grid = 2 * (total_tiles < pairs ? total_tiles : pairs);
+  const cudaError_t e = tn == 256   ? launch_pair_epi<256>(a.epilogue, s, grid, map_a, map_b, map_d, map_d2, peer_maps, p)
+                        : tn == 128 ? launch_pair_epi<128>(a.epilogue, s, grid, map_a, map_b, map_d, map_d2, peer_maps, p)
+                                    : launch_pair_epi<64>(a.epilogue, s, grid, map_a, map_b, map_d, map_d2, peer_maps, p);
+  if (e != cudaSuccess) return static_cast<int>(e);
   return finish_launch(1);
 }
 CS_DEFINE_BOUNDS_GETTER(bounds_report_gemm)
