@@ -154,10 +154,13 @@ std::array<at::Tensor, 3> attention_backward_body(const at::Tensor &dout4, const
     return {std::get<0>(r).transpose(1, 2), std::get<1>(r).transpose(1, 2), std::get<2>(r).transpose(1, 2)};
   }
   if (library_flash_ok(q)) {
+    // this library's own forward draws no random numbers and leaves the generator state undefined
+    const auto state = [&](const ReadOnlyTensor &t) {
+      return own_forward ? at::zeros({}, q.options().dtype(at::kLong)) : t.impl()->tensor;
+    };
     auto r = at::_scaled_dot_product_flash_attention_backward(
         dout.to(q.scalar_type()), q, k, v, out, lse, bw.cum_seq_q.impl()->tensor, bw.cum_seq_k.impl()->tensor,
-        bw.max_q, bw.max_k, args.dropout_p, args.is_causal, bw.philox_seed.impl()->tensor,
-        bw.philox_offset.impl()->tensor, scale);
+        bw.max_q, bw.max_k, args.dropout_p, args.is_causal, state(bw.philox_seed), state(bw.philox_offset), scale);
     return {std::get<0>(r).transpose(1, 2), std::get<1>(r).transpose(1, 2), std::get<2>(r).transpose(1, 2)};
   }
   auto r = sdpa_math_backward(dout, q, k, v, out, lse, args.is_causal, scale);
@@ -258,8 +261,8 @@ Tensor ScaledDotProductAttention::forward_packed(const Scheduler &scheduler, con
                saved.cum_k.impl()->tensor = at::Tensor{};
                state->backward.max_q = T;
                state->backward.max_k = T;
-               saved.seed.impl()->tensor = at::zeros({}, x.options().dtype(at::kLong));
-               saved.offset.impl()->tensor = at::zeros({}, x.options().dtype(at::kLong));
+               saved.seed.impl()->tensor = at::Tensor{};  // made in backward where a library engine asks for them
+               saved.offset.impl()->tensor = at::Tensor{};
                saved.out.impl()->companion = at::empty({0}, x.options());  // marks "own forward"
                output.impl()->tensor = o;
                return;
