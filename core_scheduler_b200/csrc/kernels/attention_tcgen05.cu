@@ -39,7 +39,7 @@ constexpr int THREADS = 192;
 constexpr int FWD_CTAS_PER_SM = 2;
 constexpr int FWD_STAGES = 2;
 constexpr int SMEM_BYTES = TILE_BYTES + FWD_STAGES * 2 * TILE_BYTES + 1024 + 256;  // ~81 KB
-constexpr int TMEM_COLS = 256;  // forward: S 128, P 64, O 64; backward: S', dP' and two accumulators of 64 columns each
+constexpr int TMEM_COLS = 256;  // S 128, P 64, O 64
 constexpr long long kWaitBudgetCycles = 4000000000LL;
 
 __device__ DeviceStatus g_attn_status;
@@ -77,6 +77,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
 }
+// One lane of the (converged) warp. The branch it guards must stay free of further branches: with one inside, every
+// tcgen05.mma in it takes 85 cycles to issue instead of the 34-64 it executes in.
 __device__ __forceinline__ bool elect_one() {
   uint32_t ok;
   asm volatile(
@@ -191,6 +193,15 @@ __device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t *>(&t);
+}
+
+// Bits `first` .. 31 of a 32-column mask, for any `first`.
+__device__ __forceinline__ uint32_t columns_from(int first) { return first >= 32 ? 0u : (first <= 0 ? ~0u : ~0u << first); }
+// Scores outside the mask become -inf. Bit tests on one register cost half of what 32 index comparisons do.
+__device__ __forceinline__ void mask_columns(uint32_t (&v)[32], uint32_t keep) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (!((keep >> i) & 1u)) v[i] = 0xff800000u;
 }
 
 struct AttnParams {
@@ -352,9 +363,7 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS_PER_SM) attention_fwd_kernel
       if (lane == 0) mbar_arrive(bar(S_EMPTY));
       if (p.causal && j == qb) {  // the diagonal block: key i of it is visible from row i on
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[c][i] = c * 32 + i <= r ? v[c][i] : 0xff800000u;
+        for (int c = 0; c < 4; ++c) mask_columns(v[c], ~columns_from(r + 1 - c * 32));
       }
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -458,25 +467,29 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS_PER_SM) attention_fwd_kernel
 // dQ, dK, dV of attention from the packed qkv, the forward output, its gradient and the per-row log-sum-exp; results go
 // straight into the packed dqkv [B, T, 3, H, 64].
 //
-// Three launches: (1) per-row constants, delta[b,h,t] = sum_d dO*O; (2) kDKV = true: one CTA per 128-key block keeps
-// K_j, V_j resident and streams 64-query tiles (Q_i, dO_i), accumulating dV_j and dK_j in TMEM; (3) kDKV = false: one CTA
-// per 128-query block keeps Q_i, dO_i resident and streams 64-key tiles (K_j, V_j), accumulating dQ_i in TMEM. No atomics,
+// Three launches: (1) per-row constants, delta[b,h,t] = sum_d dO*O; (2) kDKV = true: a 128-key block keeps K_j, V_j
+// resident and streams 64-query tiles (Q_i, dO_i), accumulating dV_j and dK_j in TMEM; (3) kDKV = false: a 128-query
+// block keeps Q_i, dO_i resident and streams 64-key tiles (K_j, V_j), accumulating dQ_i in TMEM. No atomics,
 // deterministic. Per streamed tile:
 //   S' = R1 C1^T, dP' = R2 C2^T              (128 x 64 x 64 each, fp32 in TMEM; rows = resident side)
 //   P' = exp(scale S' - lse), dS' = P' (dP' - delta)   (softmax warps; the factor `scale` of dS is applied to dK and dQ)
-//   [dV += P' C2]   acc += dS' C1            (128 x 64 x 64; P' and dS' stay in TMEM as bf16 A operands, C as MN-major
-//                                             operands)
-// With N = 64 an MMA reads its A operand from shared memory as often as it computes: four products with both operands
-// there move 96 KB a step, 768 cycles at 128 bytes a cycle, and writing P' and dS' there another 256, against 512 cycles
-// of tensor-core work and 512 of the exponential unit. With P' and dS' in TMEM 64 KB are left. The dK/dV kernel uses
-// all of its 256 columns, so P' and dS' lie over S' and dP' and the next scores follow the accumulating MMAs; its second
-// CTA on the SM fills that gap. The dQ kernel has room for dS' beside S' and dP'. 16 x 1024 tokens, 12 heads, causal:
-// dK/dV 138 -> BWD_DKV us, dQ 91 -> BWD_DQ us.
+//   [dV += P' C2]   acc += dS' C1            (128 x 64 x 64; P' and dS' stay in TMEM as bf16 A operands over S' and dP',
+//                                             C as MN-major operands)
+// One persistent CTA per SM owns all 512 TMEM columns: three score buffers of 128 columns and the accumulators. Three
+// groups of four softmax warps take the tiles in turn, a buffer each. What a tile costs besides its exponentials (barriers,
+// TMEM latency, the MMAs before and after it: about 1200 cycles) overlaps with the other groups' tiles, which leaves a tile
+// bound by 640 cycles of tensor core (dK/dV; 512 for dQ) or 512 of the exponential unit. All sixteen warps on one 128-column
+// tile, the score buffer of the next one ready, ran in step with each other and needed 2250 cycles for 128 columns, two CTAs
+// an SM with 64-column tiles 2800. The accumulators are drained by four warps of their own while the next block is under
+// way, across whose boundary the pipeline runs on; resident tiles are double-buffered. 16 x 1024 tokens, 12 heads, causal:
+// dK/dV 138 -> 78 us, dQ 91 -> 59; 2 x 4096, 20 heads 343 -> 164 and 231 -> 135.
 constexpr int BC = 64;                          // streamed rows per step
 constexpr int C_TILE_BYTES = BC * HD * 2;       // 8 KB
-constexpr int BWD_STAGES = 4;                   // streamed-tile stages
-constexpr int BWD_THREADS = 320;  // TMA warp, MMA warp, eight softmax warps (two threads per row: 32 columns each)
-constexpr int BWD_SMEM_BYTES = 2 * TILE_BYTES + BWD_STAGES * (2 * C_TILE_BYTES + 512) + 1024 + 256;  // ~99 KB
+constexpr int BWD_GROUPS = 3;                   // softmax groups and score buffers
+constexpr int BWD_STAGES = 6;                   // streamed-tile stages: two tiles and 512 bytes of row constants each
+constexpr int BWD_THREADS = 128 + (BWD_GROUPS + 1) * 128;  // TMA warp, two MMA warps, one idle; softmax groups, accumulator group
+constexpr int BWD_SMEM_BYTES = 4 * TILE_BYTES + BWD_STAGES * (2 * C_TILE_BYTES + 512) + 1024 + 512;  // ~165 KB
+constexpr int BWD_TMEM_COLS = 512;
 
 struct AttnBwdParams {
   __nv_bfloat16 *dqkv;     // [B, T, 3, H, 64]
@@ -534,55 +547,73 @@ __global__ void __launch_bounds__(256) attention_delta_kernel(const __nv_bfloat1
   }
 }
 
+// One 128-row block of one head: what a CTA works on at a time.
+struct BwdItem {
+  int b, h, r0, c_first, n_iter;
+};
 template <bool kDKV>
-__global__ void __launch_bounds__(BWD_THREADS, 2)
+__device__ __forceinline__ BwdItem bwd_item(const AttnBwdParams &p, int id) {
+  // Longest loops of every head first: key block 0 streams all queries, query block T/128-1 streams all keys.
+  const int heads = p.B * p.H, blocks = p.T / 128;
+  const int order = id / heads, bh = id - order * heads;
+  const int rb = kDKV ? order : blocks - 1 - order;
+  BwdItem it;
+  it.b = bh / p.H;
+  it.h = bh - it.b * p.H;
+  it.r0 = rb * 128;
+  it.c_first = kDKV && p.causal ? 2 * rb : 0;  // streamed tiles: queries r0 .. T (kDKV) or keys 0 .. r0+128
+  it.n_iter = kDKV ? 2 * blocks - it.c_first : 2 * (p.causal ? rb + 1 : blocks);
+  return it;
+}
+// The k-th block of this CTA. Blocks come in order of falling length and are dealt out back and forth, so that no CTA gets
+// the longest one of every round.
+__device__ __forceinline__ int bwd_deal(int k) { return k * gridDim.x + ((k & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x); }
+
+template <bool kDKV>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_constant__ CUtensorMap qkv_c,
                      const __grid_constant__ CUtensorMap do_r, const __grid_constant__ CUtensorMap do_c, const AttnBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *aligned = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t r1_smem = base;                      // resident operand of S'
-  const uint32_t r2_smem = r1_smem + TILE_BYTES;      // resident operand of dP'
-  const uint32_t c_smem = r2_smem + TILE_BYTES;       // per stage: C1 tile, C2 tile
-  constexpr int STAGES = BWD_STAGES;
+  constexpr int STAGES = BWD_STAGES, GROUPS = BWD_GROUPS;
+  const uint32_t r_smem = base;                            // two buffers of the resident operands of S' and dP'
+  const uint32_t c_smem = r_smem + 4 * TILE_BYTES;         // per stage: C1 tile, C2 tile
   const uint32_t vec_smem = c_smem + STAGES * 2 * C_TILE_BYTES;  // per stage: -lse[64], -delta[64] of the streamed queries
   const uint32_t bar_base = vec_smem + STAGES * 512;
   uint64_t *bars = reinterpret_cast<uint64_t *>(aligned + (bar_base - base));
-  enum { R_FULL = 0, SDP_FULL, SDP_EMPTY, PDS_FULL, PDS_EMPTY, ACC_FULL, C_FULL, C_EMPTY = C_FULL + STAGES, NUM_BARS = C_EMPTY + STAGES };
+  enum { R_FULL = 0, R_EMPTY = 2, ACC_FULL = 4, ACC_EMPTY, SDP_FULL, PDS_FULL = SDP_FULL + GROUPS, PDS_EMPTY = PDS_FULL + GROUPS,
+         C_FULL = PDS_EMPTY + GROUPS,
+         C_EMPTY = C_FULL + STAGES, NUM_BARS = C_EMPTY + STAGES };
   auto bar = [&](int i) { return bar_base + 8u * i; };
   volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(bars + NUM_BARS);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + NUM_BARS + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  // Longest loops of every head first: key block 0 streams all queries, query block T/128-1 streams all keys.
-  const int heads = p.B * p.H;
-  const int order = static_cast<int>(blockIdx.x) / heads;
-  const int bh = static_cast<int>(blockIdx.x) - order * heads;
-  const int rb = kDKV ? order : p.T / 128 - 1 - order;
-  const int b = bh / p.H, h = bh - b * p.H;
-  const int r0 = rb * 128;
-  const int row_base = b * p.T;
-  // streamed 64-row tiles: queries r0 .. T (kDKV) or keys 0 .. r0+128
-  const int c_first = (kDKV && p.causal) ? 2 * rb : 0;
-  const int n_iter = kDKV ? p.T / BC - c_first : (p.causal ? 2 * (rb + 1) : p.T / BC);
+  const int items = p.B * p.H * (p.T / 128);
 
   if (threadIdx.x == 0) {
-    mbar_init(bar(R_FULL), 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(bar(R_FULL + s), 1);
+      mbar_init(bar(R_EMPTY + s), 1);
+    }
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(bar(C_FULL + s), 1);
       mbar_init(bar(C_EMPTY + s), 1);
     }
-    mbar_init(bar(SDP_FULL), 1);
-    mbar_init(bar(SDP_EMPTY), 8);  // one arrival per softmax warp
-    mbar_init(bar(PDS_FULL), 8);
-    mbar_init(bar(PDS_EMPTY), 1);
+    for (int g = 0; g < GROUPS; ++g) {
+      mbar_init(bar(SDP_FULL + g), 1);
+      mbar_init(bar(PDS_FULL + g), 4);  // one arrival per warp of the group
+      mbar_init(bar(PDS_EMPTY + g), 1);
+    }
     mbar_init(bar(ACC_FULL), 1);
+    mbar_init(bar(ACC_EMPTY), 4);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t *>(tmem_slot))),
-                 "r"(TMEM_COLS)
+                 "r"(BWD_TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -590,207 +621,253 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
   __syncthreads();
   fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  const uint32_t s_tmem = tmem_base;             // S'   64 columns
-  const uint32_t dp_tmem = tmem_base + BC;       // dP'  64 columns
-  const uint32_t acc1_tmem = tmem_base + 2 * BC; // dV (kDKV only)
-  const uint32_t acc2_tmem = tmem_base + 3 * BC; // dK or dQ
-  // bf16 A operands: the 32 streamed columns of one softmax warp become 16 packed columns. Over S' and dP' they start
-  // where that warp's own scores were, so that no warp writes what another one still reads.
-  const uint32_t ds_tmem = kDKV ? dp_tmem : acc1_tmem;
-  constexpr uint32_t kHalfStep = kDKV ? 32 : 16;
+  // buffer g: S' in 64 columns (P' later in the first 32), dP' in the next 64 (dS' later in their first 32)
+  const uint32_t acc1_tmem = tmem_base + GROUPS * 2 * BC;  // dV (kDKV only)
+  const uint32_t acc2_tmem = acc1_tmem + HD;               // dK or dQ
 
-  const int q_col = h * HD, k_col = (p.H + h) * HD, v_col = (2 * p.H + h) * HD;
   if (warp == 0) {
-    if (elect_one()) {
-      mbar_expect_tx(bar(R_FULL), 2 * TILE_BYTES);
-      tma_load_2d(r1_smem, &qkv_r, bar(R_FULL), kDKV ? k_col : q_col, row_base + r0);
-      if (kDKV)
-        tma_load_2d(r2_smem, &qkv_r, bar(R_FULL), v_col, row_base + r0);
-      else
-        tma_load_2d(r2_smem, &do_r, bar(R_FULL), q_col, row_base + r0);
-    }
-    const float *lse_row = p.neg_lse + (static_cast<long long>(b) * p.H + h) * p.T;
-    const float *delta_row = p.neg_delta + (static_cast<long long>(b) * p.H + h) * p.T;
-    int s = 0;
-    uint32_t ph = 0;
-    for (int t = 0; t < n_iter; ++t) {
-      const int c0 = (c_first + t) * BC;
-      if (!mbar_wait_warp(bar(C_EMPTY + s), ph ^ 1u, abort_flag)) break;
-      const uint32_t c1 = c_smem + s * 2 * C_TILE_BYTES, c2 = c1 + C_TILE_BYTES;
+    int s = 0, rbuf = 0;
+    uint32_t ph = 0, rph = 0;
+    bool ok = true;
+    for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
+      const BwdItem it = bwd_item<kDKV>(p, id);
+      const int q_col = it.h * HD, k_col = (p.H + it.h) * HD, v_col = (2 * p.H + it.h) * HD, row_base = it.b * p.T;
+      ok = mbar_wait_warp(bar(R_EMPTY + rbuf), rph ^ 1u, abort_flag);
+      if (!ok) break;
+      const uint32_t r1 = r_smem + rbuf * 2 * TILE_BYTES;
       if (elect_one()) {
-        if (kDKV) {
-          mbar_expect_tx(bar(C_FULL + s), 2 * C_TILE_BYTES + 512);
-          tma_load_2d(c1, &qkv_c, bar(C_FULL + s), q_col, row_base + c0);
-          tma_load_2d(c2, &do_c, bar(C_FULL + s), q_col, row_base + c0);
-          bulk_load(vec_smem + s * 512, lse_row + c0, 256, bar(C_FULL + s));
-          bulk_load(vec_smem + s * 512 + 256, delta_row + c0, 256, bar(C_FULL + s));
-        } else {
-          mbar_expect_tx(bar(C_FULL + s), 2 * C_TILE_BYTES);
-          tma_load_2d(c1, &qkv_c, bar(C_FULL + s), k_col, row_base + c0);
-          tma_load_2d(c2, &qkv_c, bar(C_FULL + s), v_col, row_base + c0);
-        }
+        mbar_expect_tx(bar(R_FULL + rbuf), 2 * TILE_BYTES);
+        tma_load_2d(r1, &qkv_r, bar(R_FULL + rbuf), kDKV ? k_col : q_col, row_base + it.r0);
+        tma_load_2d(r1 + TILE_BYTES, kDKV ? &qkv_r : &do_r, bar(R_FULL + rbuf), kDKV ? v_col : q_col, row_base + it.r0);
       }
-      if (++s == STAGES) {
-        s = 0;
-        ph ^= 1u;
+      rbuf ^= 1;
+      if (rbuf == 0) rph ^= 1u;
+      const long long vec_row = (static_cast<long long>(it.b) * p.H + it.h) * p.T;
+      for (int t = 0; t < it.n_iter; ++t) {
+        const int c0 = (it.c_first + t) * BC;
+        ok = mbar_wait_warp(bar(C_EMPTY + s), ph ^ 1u, abort_flag);
+        if (!ok) break;
+        const uint32_t c1 = c_smem + s * 2 * C_TILE_BYTES, c2 = c1 + C_TILE_BYTES;
+        if (elect_one()) {
+          if (kDKV) {
+            mbar_expect_tx(bar(C_FULL + s), 2 * C_TILE_BYTES + 512);
+            tma_load_2d(c1, &qkv_c, bar(C_FULL + s), q_col, row_base + c0);
+            tma_load_2d(c2, &do_c, bar(C_FULL + s), q_col, row_base + c0);
+            bulk_load(vec_smem + s * 512, p.neg_lse + vec_row + c0, 256, bar(C_FULL + s));
+            bulk_load(vec_smem + s * 512 + 256, p.neg_delta + vec_row + c0, 256, bar(C_FULL + s));
+          } else {
+            mbar_expect_tx(bar(C_FULL + s), 2 * C_TILE_BYTES);
+            tma_load_2d(c1, &qkv_c, bar(C_FULL + s), k_col, row_base + c0);
+            tma_load_2d(c2, &qkv_c, bar(C_FULL + s), v_col, row_base + c0);
+          }
+        }
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1u;
+        }
       }
     }
   } else if (warp == 1) {
-    // S', dP': M=128, N=64, both operands K-major. Accumulators: M=128, N=64, A from TMEM, B MN-major.
-    constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BC >> 3) << 17) | (8u << 24);
-    constexpr uint32_t idesc_a = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (static_cast<uint32_t>(HD >> 3) << 17) | (8u << 24);
-    // descriptors are built once; a k-step or a stage only advances the 16-byte-unit address field
-    const uint64_t d_r1 = smem_desc(r1_smem, 16, 1024), d_r2 = smem_desc(r2_smem, 16, 1024);
-    const uint64_t d_c1k = smem_desc(c_smem, 16, 1024), d_c2k = smem_desc(c_smem + C_TILE_BYTES, 16, 1024);
-    const uint64_t d_c1m = smem_desc(c_smem, 8192, 1024), d_c2m = smem_desc(c_smem + C_TILE_BYTES, 8192, 1024);
-    constexpr uint64_t kStage = (2 * C_TILE_BYTES) >> 4;
-    constexpr uint64_t kStepK = 32 >> 4, kStepMN = 2048 >> 4;  // 16 elements along K: 32 bytes K-major, 2 KB MN-major
-    bool ok = mbar_wait_warp(bar(R_FULL), 0, abort_flag);
-    int fs = 0;  // stage and phase of the next tile whose scores are issued
-    uint32_t fph = 0;
-    auto issue_sdp = [&](int t) -> bool {
-      if (!mbar_wait_warp(bar(C_FULL + fs), fph, abort_flag)) return false;
-      if (!kDKV && !mbar_wait_warp(bar(SDP_EMPTY), (t & 1) ^ 1u, abort_flag)) return false;
-      fence_after();
-      const uint64_t at = fs * kStage;
-      if (elect_one()) {
-#pragma unroll
-        for (int k = 0; k < HD / 16; ++k) umma(s_tmem, d_r1 + k * kStepK, d_c1k + at + k * kStepK, idesc_s, k > 0 ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < HD / 16; ++k) umma(dp_tmem, d_r2 + k * kStepK, d_c2k + at + k * kStepK, idesc_s, k > 0 ? 1u : 0u);
-        umma_commit(bar(SDP_FULL));
-      }
-      if (++fs == STAGES) {
-        fs = 0;
-        fph ^= 1u;
-      }
-      return true;
-    };
-    if (ok) ok = issue_sdp(0);
-    int t = 0, s = 0;
-    for (; ok && t < n_iter; ++t) {
-      // dQ kernel: the scores of tile t+1 are issued as soon as the softmax warps hold those of tile t in registers
-      if (!kDKV && t + 1 < n_iter) ok = issue_sdp(t + 1);
+    // S' and dP' of every tile, as soon as its buffer is free: M=128, N=64, both operands K-major
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BC >> 3) << 17) | (8u << 24);
+    // descriptors are built once; a k-step, a stage or a buffer only advances the 16-byte-unit address field
+    const uint64_t d_r1 = smem_desc(r_smem, 16, 1024), d_r2 = smem_desc(r_smem + TILE_BYTES, 16, 1024);
+    const uint64_t d_c1 = smem_desc(c_smem, 16, 1024), d_c2 = smem_desc(c_smem + C_TILE_BYTES, 16, 1024);
+    constexpr uint64_t kStage = (2 * C_TILE_BYTES) >> 4, kBuffer = (2 * TILE_BYTES) >> 4, kStepK = 32 >> 4;
+    int s = 0, g = 0, rbuf = 0;
+    uint32_t cph = 0, gph = 0, rph = 0;
+    bool ok = true;
+    for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
+      const int n_iter = bwd_item<kDKV>(p, id).n_iter;
+      ok = mbar_wait_warp(bar(R_FULL + rbuf), rph, abort_flag);
       if (!ok) break;
-      if (!mbar_wait_warp(bar(PDS_FULL), t & 1, abort_flag)) break;
-      fence_after();
-      const uint64_t at = s * kStage;
-      if (elect_one()) {
+      const uint64_t rt = rbuf * kBuffer;
+      for (int t = 0; t < n_iter; ++t) {
+        ok = mbar_wait_warp(bar(C_FULL + s), cph, abort_flag) && mbar_wait_warp(bar(PDS_EMPTY + g), gph ^ 1u, abort_flag);
+        if (!ok) break;
+        fence_after();
+        const uint64_t at = s * kStage;
+        const uint32_t s_tmem = tmem_base + g * 2 * BC;
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < BC / 16; ++k) {
-          const uint32_t a_col = (k >> 1) * kHalfStep + (k & 1) * 8;
-          if (kDKV) umma_ts(acc1_tmem, s_tmem + a_col, d_c2m + at + k * kStepMN, idesc_a, (t | k) ? 1u : 0u);
-          umma_ts(acc2_tmem, ds_tmem + a_col, d_c1m + at + k * kStepMN, idesc_a, (t | k) ? 1u : 0u);
+          for (int kk = 0; kk < HD / 16; ++kk) umma(s_tmem, d_r1 + rt + kk * kStepK, d_c1 + at + kk * kStepK, idesc, kk > 0 ? 1u : 0u);
+#pragma unroll
+          for (int kk = 0; kk < HD / 16; ++kk) umma(s_tmem + BC, d_r2 + rt + kk * kStepK, d_c2 + at + kk * kStepK, idesc, kk > 0 ? 1u : 0u);
+          umma_commit(bar(SDP_FULL + g));
         }
-        if (!kDKV) umma_commit(bar(PDS_EMPTY));
-        umma_commit(bar(C_EMPTY + s));
+        if (++s == STAGES) {
+          s = 0;
+          cph ^= 1u;
+        }
+        if (++g == GROUPS) {
+          g = 0;
+          gph ^= 1u;
+        }
       }
-      if (++s == STAGES) s = 0;
-      // dK/dV kernel: the next scores overwrite P' and dS'; MMAs execute in the order they are issued
-      if (kDKV && t + 1 < n_iter) ok = issue_sdp(t + 1);
+      if (ok && elect_one()) umma_commit(bar(R_EMPTY + rbuf));
+      rbuf ^= 1;
+      if (rbuf == 0) rph ^= 1u;
     }
-    if (ok && t == n_iter && elect_one()) umma_commit(bar(ACC_FULL));
-  } else {
-    const int q = warp & 3;            // TMEM lane quarter this warp may access
-    const int half = (warp - 2) >> 2;  // which 32 of the 64 streamed columns this thread handles
-    const int r = q * 32 + lane;       // row of the resident block
-    const int r_idx = r0 + r;
-    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
-    float lse_r = 0.f, delta_r = 0.f;
-    if (!kDKV) {
-      lse_r = p.neg_lse[(static_cast<long long>(b) * p.H + h) * p.T + r_idx];
-      delta_r = p.neg_delta[(static_cast<long long>(b) * p.H + h) * p.T + r_idx];
+  } else if (warp == 2) {
+    // accumulators: M=128, N=64, A (P', dS') from TMEM, B MN-major. A warp of its own: issuing blocks while the pipe is
+    // full, and one warp's waits for the two kinds of products cost as much as the products.
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (static_cast<uint32_t>(HD >> 3) << 17) | (8u << 24);
+    const uint64_t d_c1 = smem_desc(c_smem, 8192, 1024), d_c2 = smem_desc(c_smem + C_TILE_BYTES, 8192, 1024);
+    constexpr uint64_t kStage = (2 * C_TILE_BYTES) >> 4, kStepMN = 2048 >> 4;
+    int s = 0, g = 0;
+    uint32_t gph = 0, item_parity = 0;
+    bool ok = true;
+    for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
+      const int n_iter = bwd_item<kDKV>(p, id).n_iter;
+      ok = mbar_wait_warp(bar(ACC_EMPTY), item_parity ^ 1u, abort_flag);  // the accumulators of the block before have been read
+      item_parity ^= 1u;
+      if (!ok) break;
+      for (int t = 0; t < n_iter; ++t) {
+        ok = mbar_wait_warp(bar(PDS_FULL + g), gph, abort_flag);
+        if (!ok) break;
+        fence_after();
+        const uint64_t at = s * kStage;
+        const uint32_t p_tmem = tmem_base + g * 2 * BC, ds_tmem = p_tmem + BC;
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < BC / 16; ++kk) {
+            if (kDKV) umma_ts(acc1_tmem, p_tmem + kk * 8, d_c2 + at + kk * kStepMN, idesc, (t | kk) ? 1u : 0u);
+            umma_ts(acc2_tmem, ds_tmem + kk * 8, d_c1 + at + kk * kStepMN, idesc, (t | kk) ? 1u : 0u);
+          }
+          umma_commit(bar(PDS_EMPTY + g));
+          umma_commit(bar(C_EMPTY + s));
+        }
+        if (++s == STAGES) s = 0;
+        if (++g == GROUPS) {
+          g = 0;
+          gph ^= 1u;
+        }
+      }
+      if (ok && elect_one()) umma_commit(bar(ACC_FULL));
     }
-    const F2 scale2 = f2(p.scale_log2e, p.scale_log2e), lse_r2 = f2(lse_r, lse_r), delta_r2 = f2(delta_r, delta_r);
-    int s = 0;
-    uint32_t cph = 0;
-    for (int t = 0; t < n_iter; ++t) {
-      const int c0 = (c_first + t) * BC + half * 32;  // first streamed row of this thread
-      if (kDKV && !mbar_wait_warp(bar(C_FULL + s), cph, abort_flag)) break;  // -lse / -delta of the streamed queries
-      if (!mbar_wait_warp(bar(SDP_FULL), t & 1, abort_flag)) break;
-      fence_after();
-      uint32_t sv[32], dv[32];
-      tmem_ld32(s_tmem + half * 32 + lane_addr, sv);
-      tmem_ld32(dp_tmem + half * 32 + lane_addr, dv);
-      tmem_wait_ld();
-      if (!kDKV) {  // S' and dP' of this tile live in registers: the tensor core may overwrite them with the next tile's
+  } else if (warp >= 4 && warp < 4 + 4 * GROUPS) {
+    const int q = warp & 3;          // TMEM lane quarter this warp may access
+    const int g = (warp - 4) >> 2;   // softmax group: tiles g, g + GROUPS, ...
+    const int r = q * 32 + lane;     // row of the resident block
+    const uint32_t s_tmem = tmem_base + g * 2 * BC + (static_cast<uint32_t>(q * 32) << 16), dp_tmem = s_tmem + BC;
+    const F2 scale2 = f2(p.scale_log2e, p.scale_log2e);
+    int next = g;        // steps until this group's next tile, counted from the start of a block
+    int s = g;           // stage of that tile
+    uint32_t cph = 0, parity = 0;
+    bool ok = true;
+    for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
+      const BwdItem it = bwd_item<kDKV>(p, id);
+      if (next >= it.n_iter) {
+        next -= it.n_iter;
+        continue;
+      }
+      float lse_r = 0.f, delta_r = 0.f;
+      if (!kDKV) {
+        const long long at = (static_cast<long long>(it.b) * p.H + it.h) * p.T + it.r0 + r;
+        lse_r = p.neg_lse[at];
+        delta_r = p.neg_delta[at];
+      }
+      const F2 lse_r2 = f2(lse_r, lse_r), delta_r2 = f2(delta_r, delta_r);
+      for (; next < it.n_iter; next += GROUPS) {
+        if (kDKV) {
+          ok = mbar_wait_warp(bar(C_FULL + s), cph, abort_flag);  // -lse / -delta of the streamed queries
+          if (!ok) break;
+        }
+        ok = mbar_wait_warp(bar(SDP_FULL + g), parity, abort_flag);
+        if (!ok) break;
+        parity ^= 1u;
+        fence_after();
+        const int c0 = (it.c_first + next) * BC - it.r0;  // first streamed row, relative to the resident block
+        // rows are keys and columns queries (kDKV), or rows queries and columns keys: keep key <= query
+        const bool masked = p.causal && (kDKV ? c0 < 128 : c0 + BC > 0);
+        const uint32_t vec = vec_smem + s * 512;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {  // 32 columns at a time
+          uint32_t sv[32], dv[32];
+          tmem_ld32(s_tmem + c * 32, sv);
+          tmem_ld32(dp_tmem + c * 32, dv);
+          tmem_wait_ld();
+          if (masked) {
+            const int first = r - c0 - c * 32;  // dK/dV: columns below it are masked; dQ: columns above it
+            mask_columns(sv, kDKV ? columns_from(first) : ~columns_from(first + 1));
+          }
+          uint32_t pp[16], dd[16];
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            F2 nl[2] = {lse_r2, lse_r2}, nd[2] = {delta_r2, delta_r2};
+            if (kDKV) {
+              ld_shared_pairs(vec + (c * 32 + i) * 4, nl[0], nl[1]);
+              ld_shared_pairs(vec + 256 + (c * 32 + i) * 4, nd[0], nd[1]);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const int e = i + 2 * j;
+              float a, d;
+              f2_split(f2_fma(f2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), scale2, nl[j]), a, d);
+              const F2 pr = f2(fast_exp2(a), fast_exp2(d));
+              const F2 ds = f2_mul(pr, f2_add(f2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), nd[j]));
+              if (kDKV) {
+                f2_split(pr, a, d);
+                pp[e >> 1] = pack2(a, d);
+              }
+              f2_split(ds, a, d);
+              dd[e >> 1] = pack2(a, d);
+            }
+          }
+          // over the scores of columns 0..31, which this warp has read
+          if (kDKV) tmem_st16(s_tmem + c * 16, pp);
+          tmem_st16(dp_tmem + c * 16, dd);
+        }
+        tmem_wait_st();
         fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(SDP_EMPTY));
-      }
-      uint32_t pp[16], dd[16];
-      const uint32_t vec = vec_smem + s * 512 + half * 128;
-#pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        F2 nl[2] = {lse_r2, lse_r2}, nd[2] = {delta_r2, delta_r2};
-        if (kDKV) {
-          ld_shared_pairs(vec + i * 4, nl[0], nl[1]);
-          ld_shared_pairs(vec + 256 + i * 4, nd[0], nd[1]);
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int e = i + 2 * j;
-          float a, d;
-          f2_split(f2_fma(f2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), scale2, nl[j]), a, d);
-          const F2 pr = f2(fast_exp2(a), fast_exp2(d));
-          const F2 ds = f2_mul(pr, f2_add(f2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), nd[j]));
-          if (kDKV) {
-            f2_split(pr, a, d);
-            pp[e >> 1] = pack2(a, d);
-          }
-          f2_split(ds, a, d);
-          dd[e >> 1] = pack2(a, d);
+        if (lane == 0) mbar_arrive(bar(PDS_FULL + g));
+        s += GROUPS;
+        if (s >= STAGES) {
+          s -= STAGES;
+          cph ^= 1u;
         }
       }
-      // rows are keys and columns queries (kDKV), or rows queries and columns keys: keep key <= query
-      if (p.causal && (kDKV ? c0 < r0 + q * 32 + 31 : c0 + 31 > r0 + q * 32)) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int col = c0 + 2 * i;
-          const uint32_t keep = ((kDKV ? r_idx <= col : col <= r_idx) ? 0x0000ffffu : 0u) |
-                                ((kDKV ? r_idx <= col + 1 : col + 1 <= r_idx) ? 0xffff0000u : 0u);
-          if (kDKV) pp[i] &= keep;
-          dd[i] &= keep;
-        }
-      }
-      if (!kDKV && !mbar_wait_warp(bar(PDS_EMPTY), (t & 1) ^ 1u, abort_flag)) break;  // tile t-1's dQ MMA has read dS'
-      if (kDKV) tmem_st16(s_tmem + half * kHalfStep + lane_addr, pp);
-      tmem_st16(ds_tmem + half * kHalfStep + lane_addr, dd);
-      tmem_wait_st();
-      fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(PDS_FULL));
-      if (++s == STAGES) {
-        s = 0;
-        cph ^= 1u;
-      }
+      next -= it.n_iter;
     }
-    if (mbar_wait_warp(bar(ACC_FULL), 0, abort_flag) && !*abort_flag) {
+  } else if (warp >= 4 + 4 * GROUPS) {
+    // accumulators -> dqkv: thread = row; dV and dK, or dQ
+    const int q = warp & 3;
+    const int r = q * 32 + lane;
+    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    uint32_t parity = 0;
+    for (int k = 0, id; (id = bwd_deal(k)) < items; ++k) {
+      const BwdItem it = bwd_item<kDKV>(p, id);
+      if (!mbar_wait_warp(bar(ACC_FULL), parity, abort_flag)) break;
+      parity ^= 1u;
       fence_after();
-      const long long row = static_cast<long long>(row_base + r_idx) * 3 * p.H;
+      const long long row = static_cast<long long>(it.b * p.T + it.r0 + r) * 3 * p.H;
       const bool row_in_range =
-          CS_IN_BOUNDS(kKidAttention, (row + 2LL * p.H + h) * HD + HD - 1, static_cast<long long>(p.B) * p.T * 3 * p.H * HD);
-      auto store = [&](uint32_t tmem, int part, float factor) {
-        __nv_bfloat16 *dst = p.dqkv + (row + static_cast<long long>(part) * p.H + h) * HD + half * 32;
-        uint32_t v[32];
-        tmem_ld32(tmem + half * 32 + lane_addr, v);
-        tmem_wait_ld();
-        if (!row_in_range) return;
+          CS_IN_BOUNDS(kKidAttention, (row + 2LL * p.H + it.h) * HD + HD - 1, static_cast<long long>(p.B) * p.T * 3 * p.H * HD);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 w;
-          w.x = pack2(__uint_as_float(v[g * 8 + 0]) * factor, __uint_as_float(v[g * 8 + 1]) * factor);
-          w.y = pack2(__uint_as_float(v[g * 8 + 2]) * factor, __uint_as_float(v[g * 8 + 3]) * factor);
-          w.z = pack2(__uint_as_float(v[g * 8 + 4]) * factor, __uint_as_float(v[g * 8 + 5]) * factor);
-          w.w = pack2(__uint_as_float(v[g * 8 + 6]) * factor, __uint_as_float(v[g * 8 + 7]) * factor);
-          *reinterpret_cast<uint4 *>(dst + g * 8) = w;
+      for (int part = kDKV ? 0 : 2; part < 4; ++part) {  // 32 columns each: dV, dV, dK (dQ), dK (dQ)
+        const int which = kDKV ? (part < 2 ? 2 : 1) : 0;
+        const float factor = part < 2 ? 1.f : p.scale;
+        uint32_t v[32];
+        tmem_ld32((part < 2 ? acc1_tmem : acc2_tmem) + (part & 1) * 32 + lane_addr, v);
+        tmem_wait_ld();
+        if (part == 3) {
+          fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(ACC_EMPTY));
         }
-      };
-      if (kDKV) {
-        store(acc1_tmem, 2, 1.f);      // dV
-        store(acc2_tmem, 1, p.scale);  // dK
-      } else {
-        store(acc2_tmem, 0, p.scale);  // dQ
+        __nv_bfloat16 *dst = p.dqkv + (row + static_cast<long long>(which) * p.H + it.h) * HD + (part & 1) * 32;
+        if (row_in_range) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            uint4 w;
+            w.x = pack2(__uint_as_float(v[i * 8 + 0]) * factor, __uint_as_float(v[i * 8 + 1]) * factor);
+            w.y = pack2(__uint_as_float(v[i * 8 + 2]) * factor, __uint_as_float(v[i * 8 + 3]) * factor);
+            w.z = pack2(__uint_as_float(v[i * 8 + 4]) * factor, __uint_as_float(v[i * 8 + 5]) * factor);
+            w.w = pack2(__uint_as_float(v[i * 8 + 6]) * factor, __uint_as_float(v[i * 8 + 7]) * factor);
+            *reinterpret_cast<uint4 *>(dst + i * 8) = w;
+          }
+        }
       }
     }
   }
@@ -805,7 +882,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
   }
   if (warp == 1) {
     fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(BWD_TMEM_COLS) : "memory");
   }
 }
 
@@ -924,7 +1001,14 @@ int attention_backward_packed(stream_t stream, const void *qkv, const void *out,
   p.scale_log2e = scale * 1.4426950408889634f;
   p.status = attn_status_ptr();
   p.causal = causal ? 1 : 0;
-  const auto grid = static_cast<unsigned>(T / 128 * H * B);
+  const int64_t items = T / 128 * H * B;
+  static const int sm_count = [] {
+    int dev = 0, n = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+  }();
+  const auto grid = static_cast<unsigned>(items < sm_count ? items : sm_count);
   attention_bwd_kernel<true><<<grid, BWD_THREADS, BWD_SMEM_BYTES, s>>>(qkv_r, qkv_c, do_r, do_c, p);
   attention_bwd_kernel<false><<<grid, BWD_THREADS, BWD_SMEM_BYTES, s>>>(qkv_r, qkv_c, do_r, do_c, p);
   return finish_launch(3);

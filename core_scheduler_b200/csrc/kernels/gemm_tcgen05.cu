@@ -111,8 +111,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // The tensor-core and TMA instructions take their operands from uniform registers. In a branch that one lane took on its own
 // (`if (lane == 0)`) the compiler has to move every operand there again for each instruction: 79 cycles an MMA and 220
 // cycles a k-block of TMA loads were measured, more than the tensor core needs for a tile of 128 columns. So a role's whole
-// warp walks its loop in step and elects a lane only around the instructions themselves; waits are voted on, which keeps
-// the control flow uniform when one of them is abandoned.
+// warp walks its loop in step and elects a lane only around the instructions themselves, without another branch inside
+// (one there brings the 85 cycles back); waits are voted on, which keeps the control flow uniform when one is abandoned.
 __device__ __forceinline__ bool elect_one() {
   uint32_t ok;
   asm volatile(
@@ -704,17 +704,22 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         const uint32_t a_dst = smem_base + stage * STAGE2_BYTES;
         const uint32_t b_dst = a_dst + A_BYTES;
         const uint32_t full_leader = mapa_shared(full_bar(stage), 0);
-        if (elect_one()) {
-          if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE2_BYTES);
-          if (p.layout == kNT) {
+        if (leader && elect_one()) mbar_expect_tx(full_bar(stage), 2 * STAGE2_BYTES);
+        if (p.layout == kTN) {
+          if (elect_one()) {
+            tma_load_2d_pair(a_dst, rows_map, full_leader, kb * BK, row);
+            tma_load_2d_pair(b_dst, &map_b, full_leader, kb * BK, nb0);
+          }
+        } else if (p.layout == kNT) {
+          if (elect_one()) {
 #pragma unroll
             for (int j = 0; j < 2; ++j) tma_load_2d_pair(a_dst + j * 8192, &map_a, full_leader, m0 + j * 64, kb * BK);
-          } else {
-            tma_load_2d_pair(a_dst, rows_map, full_leader, kb * BK, row);
+#pragma unroll
+            for (int j = 0; j < TN / 128; ++j) tma_load_2d_pair(b_dst + j * 8192, &map_b, full_leader, nb0 + j * 64, kb * BK);
           }
-          if (p.layout == kTN) {
-            tma_load_2d_pair(b_dst, &map_b, full_leader, kb * BK, nb0);
-          } else {
+        } else {
+          if (elect_one()) {
+            tma_load_2d_pair(a_dst, rows_map, full_leader, kb * BK, row);
 #pragma unroll
             for (int j = 0; j < TN / 128; ++j) tma_load_2d_pair(b_dst + j * 8192, &map_b, full_leader, nb0 + j * 64, kb * BK);
           }
@@ -760,8 +765,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             for (int k = 0; k < BK / UMMA_K; ++k)
               tcgen05_mma_pair(d_tmem, da + k * kstep_a, db + k * kstep_b, idesc, (kb > c.kb_begin || k > 0) ? 1u : 0u);
             tcgen05_commit_pair(empty_bar(stage));
-            if (kb + 1 == c.kb_end) tcgen05_commit_pair(tmem_full_bar(acc));
           }
+          if (kb + 1 == c.kb_end && elect_one()) tcgen05_commit_pair(tmem_full_bar(acc));
           if (++stage == STAGES2) {
             stage = 0;
             phase ^= 1u;

@@ -125,3 +125,32 @@ def test_non_causal_attention_through_the_op_stays_on_own_kernels(gpu_scheduler)
     assert C.kernel_launch_count() - before == 1 and C.library_fallbacks() == fallbacks
     q, k, v = qkv.float().view(B, T, 3, H, D).unbind(2)
     assert torch.allclose(out.raw().float(), attention_reference(q, k, v, causal=False).reshape(B, T, H * D), atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("B,T,H", [(5, 384, 13), (2, 1024, 12), (1, 2176, 9), (149, 128, 1)])
+def test_blocks_dealt_to_persistent_ctas(B, T, H, causal):
+    """More 128-row blocks than SMs, an odd number of them and of tiles in each: the backward pipeline runs across block
+    boundaries. Keys grow along the sequence, so that the forward pass has to move its reference maximum more than once.
+    P, dS and the results are rounded to bf16 (2^-9 each); in the 2-norm of a gradient that stays below 1e-2."""
+    D = 64
+    torch.manual_seed(B + T + H)
+    qkv = torch.randn(B, T, 3, H, D, device="cuda")
+    qkv[:, :, 1] *= torch.linspace(0.3, 4.0, T, device="cuda")[None, :, None, None]
+    qkv = qkv.view(B, T, 3 * H * D).to(BF)
+    dout = torch.randn(B, T, H * D, device="cuda").to(BF)
+    rc, out, lse = C.attention_forward_tcgen05(qkv, H, 0.125, causal=causal)
+    assert rc == 0
+    dqkv, _ = C.attention_backward_tcgen05(qkv, out, dout, lse, H, 0.125, causal=causal)
+    again, _ = C.attention_backward_tcgen05(qkv, out, dout, lse, H, 0.125, causal=causal)
+    torch.cuda.synchronize()
+    assert C.attention_status()[0] == 0
+    assert torch.equal(dqkv, again)  # no atomics: the same bits every time
+    qr = qkv.double().requires_grad_(True)
+    q, k, v = qr.view(B, T, 3, H, D).unbind(2)
+    ref = attention_reference(q, k, v, causal=causal).reshape(B, T, H * D)
+    ref.backward(dout.double())
+    assert ((out.double() - ref).norm() / ref.norm()).item() < 6e-3
+    got, want = dqkv.double().view(B, T, 3, H, D), qr.grad.view(B, T, 3, H, D)
+    for i in range(3):
+        assert ((got[:, :, i] - want[:, :, i]).norm() / want[:, :, i].norm()).item() < 1e-2
