@@ -293,3 +293,26 @@ def test_gpt2_bf16_training_matches_fp32_autograd_and_library_backend(gpu_schedu
         g, r = grads[k].float(), ref.p(k).grad
         err = (g - r).norm() / (r.norm() + 1e-12)
         assert err < 5e-2, (k, err.item())
+
+
+@pytest.mark.parametrize("rows,d,offset", [(1, 8, 0), (50, 768, 0), (333, 1000, 0), (64, 264, 1)])
+def test_embedding_backward_hot_ids_and_unaligned_table(gpu_scheduler, rows, d, offset):
+    """Most rows add into one id; the gradient table starts at any fp32 element (vector or scalar reductions). Up to `rows` fp32
+    additions in any order: an error of rows * 2^-24 of the largest partial sum."""
+    s = gpu_scheduler
+    torch.manual_seed(rows + d)
+    V = 40
+    te = C.embedding_init(s, V, d)
+    idx = torch.randint(0, V, (rows,), device="cuda")
+    idx[: rows // 2 + 1] = 7
+    dy = torch.randn(rows, d, device="cuda").to(BF)
+    store = torch.zeros(V * d + offset, device="cuda")
+    te.grad_weight.set_raw(store[offset:].view(V, d))
+    with cs.autocast(s, BF):
+        y = C.embedding_forward(s, te, T(idx))
+    C.embedding_backward(s, te, T(dy))
+    s.synchronize()
+    assert torch.equal(y.raw(), te.weight.raw()[idx].to(BF))
+    want = torch.zeros(V, d, device="cuda", dtype=torch.float64).index_add_(0, idx, dy.double())
+    bound = rows * 2.0 ** -24 * torch.zeros(V, d, device="cuda", dtype=torch.float64).index_add_(0, idx, dy.double().abs()).max()
+    assert (te.grad_weight.raw().double() - want).abs().max() <= bound
