@@ -316,3 +316,30 @@ def test_embedding_backward_hot_ids_and_unaligned_table(gpu_scheduler, rows, d, 
     want = torch.zeros(V, d, device="cuda", dtype=torch.float64).index_add_(0, idx, dy.double())
     bound = rows * 2.0 ** -24 * torch.zeros(V, d, device="cuda", dtype=torch.float64).index_add_(0, idx, dy.double().abs()).max()
     assert (te.grad_weight.raw().double() - want).abs().max() <= bound
+
+
+@pytest.mark.parametrize("rows,d", [(1, 8), (3, 256), (5, 264), (4099, 760), (2500, 1600), (1030, 2048), (2, 2056)])
+def test_layernorm_column_kernels(gpu_scheduler, rows, d):
+    """Widths around a warp's 256 columns and the 2048 limit, row counts around the group of four, more rows than one wave of
+    CTAs, and the accumulation into existing gradients. bf16 outputs: half an ulp, 2^-9; fp32 sums over the rows: 1e-5."""
+    s = gpu_scheduler
+    torch.manual_seed(rows + d)
+    st = C.layer_norm_init(s, [d])
+    st.weight.raw().uniform_(0.5, 1.5)
+    st.bias.raw().uniform_(-0.5, 0.5)
+    x, dy, res = (torch.randn(rows, d, device="cuda").mul_(2).add_(0.5).to(BF) for _ in range(3))
+    xr = x.double().requires_grad_(True)
+    w, b = (t.raw().double().requires_grad_(True) for t in (st.weight, st.bias))
+    yr = F.layer_norm(xr, (d,), w, b)
+    yr.backward(dy.double())
+
+    def rel(a, want):
+        return ((a.double() - want).norm() / want.norm()).item()
+
+    for step in (1, 2):
+        with cs.autocast(s, BF):
+            y = C.layer_norm_forward(s, st, T(x))
+        dx = C.layer_norm_backward(s, st, T(dy), T(res))
+        s.synchronize()
+        assert rel(y.raw(), yr.detach()) < 2e-3 and rel(dx.raw(), xr.grad + res.double()) < 3e-3
+        assert rel(st.grad_weight.raw(), step * w.grad) < 1e-5 and rel(st.grad_bias.raw(), step * b.grad) < 1e-5
