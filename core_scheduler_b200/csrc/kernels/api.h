@@ -159,6 +159,10 @@ int cross_entropy_finalize(stream_t stream, const float *stats, int64_t n_tiles,
 int cross_entropy_backward_inplace(stream_t stream, void *logits, int64_t ld, const float *lse,
                                    const int64_t *target, const float *count, float grad_scale, int64_t rows,
                                    int64_t n, int64_t n_valid, int64_t ignore_index, int64_t col_offset = 0);
+// out[n] (+)= sums of the columns of the contiguous bf16 matrix x [rows, n]; n % 8 == 0, x 16-byte aligned. `scratch` holds
+// column_sum_parts(rows, n) * n floats (unused when that is one part).
+int64_t column_sum_parts(int64_t rows, int64_t n);
+int column_sum(stream_t stream, const void *x, int64_t rows, int64_t n, float *out, int accumulate, float *scratch);
 // Per-row statistics of one vocabulary slice (classes [col_offset, col_offset + ld)): out[row] = (log-sum-exp over
 // the slice's valid columns from the GEMM's per-tile partials, or -inf when it has none; the target's logit when the
 // target class falls into the slice's first n_valid_local columns, else 0).

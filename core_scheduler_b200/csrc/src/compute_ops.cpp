@@ -325,8 +325,28 @@ void linear_wgrad(const at::Tensor &dy_in, const at::Tensor &x_in, at::ScalarTyp
   store_grad(grad_slot, at::matmul(dy2.t(), x2), store);
 }
 
-void bias_grad(const at::Tensor &dy, const Tensor &bias, const Tensor &grad_slot) {
+void bias_grad(const at::Tensor &dy, const Tensor &bias, const Tensor &grad_slot, const FnTask &task) {
   const at::ScalarType store = bias.impl()->tensor.scalar_type();
+  if (dy.is_cuda() && dy.scalar_type() == at::kBFloat16 && dy.is_contiguous() && fused_enabled() && store == at::kFloat &&
+      dy.numel() > 0 && dy.size(-1) % 8 == 0 && (reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15) == 0) {
+    auto &slot = *grad_slot.impl();
+    const bool had = slot.tensor.defined();
+    if (!had || grad_slot_ready_for_fused(grad_slot)) {
+      const int64_t n = dy.size(-1), rows = dy.numel() / n;
+      if (!had) slot.tensor = at::empty({n}, dy.options().dtype(at::kFloat));
+      const int64_t parts = kernels::column_sum_parts(rows, n);
+      at::Tensor scratch;
+      if (parts > 1) {
+        scratch = at::empty({parts * n}, dy.options().dtype(at::kFloat));
+        task.intermediate().push_back(scratch);
+      }
+      check_kernel(kernels::column_sum(current_stream(), dy.data_ptr(), rows, n, slot.tensor.data_ptr<float>(), had && !slot.fresh ? 1 : 0,
+                                       parts > 1 ? scratch.data_ptr<float>() : nullptr),
+                   "column_sum");
+      slot.fresh = false;
+      return;
+    }
+  }
   const at::Tensor dy2 = dy.reshape({-1, dy.size(-1)});
   store_grad(grad_slot, at::sum(dy2, {0}, false, store == at::kDouble ? at::kDouble : at::kFloat).to(store), store);
 }
@@ -407,8 +427,8 @@ void Linear::backward_parameter(const Scheduler &scheduler, const std::shared_pt
   if (state->args.bias) {
     submit(scheduler, "cs::compute::Linear::backward_bias", Task::Impl::kAssist, Task::Impl::kCompute,
            {state->forward.grad_bias}, {grad_output, state->forward.bias},
-           [grad_output, b = state->forward.bias, gb = state->forward.grad_bias](const FnTask &) {
-             bias_grad(grad_output.impl()->tensor, b, gb);
+           [grad_output, b = state->forward.bias, gb = state->forward.grad_bias](const FnTask &task) {
+             bias_grad(grad_output.impl()->tensor, b, gb, task);
            });
   }
   state->backward.input.reset();  // the tasks hold their own references
@@ -516,8 +536,8 @@ void GeluLinear::backward_parameter(const Scheduler &scheduler, const std::share
   if (state->args.bias) {
     submit(scheduler, "cs::compute::GeluLinear::backward_bias", Task::Impl::kAssist, Task::Impl::kCompute,
            {state->forward.grad_bias}, {grad_output, state->forward.bias},
-           [grad_output, b = state->forward.bias, gb = state->forward.grad_bias](const FnTask &) {
-             bias_grad(grad_output.impl()->tensor, b, gb);
+           [grad_output, b = state->forward.bias, gb = state->forward.grad_bias](const FnTask &task) {
+             bias_grad(grad_output.impl()->tensor, b, gb, task);
            });
   }
   gelu_linear_release(state);

@@ -343,3 +343,21 @@ def test_layernorm_column_kernels(gpu_scheduler, rows, d):
         s.synchronize()
         assert rel(y.raw(), yr.detach()) < 2e-3 and rel(dx.raw(), xr.grad + res.double()) < 3e-3
         assert rel(st.grad_weight.raw(), step * w.grad) < 1e-5 and rel(st.grad_bias.raw(), step * b.grad) < 1e-5
+
+
+@pytest.mark.parametrize("rows,n", [(1, 8), (31, 72), (64, 3072), (65, 64), (3000, 5120), (70001, 136)])
+def test_bias_gradient_column_sums(gpu_scheduler, rows, n):
+    """One block per column group and several, remainders of both; stored, then accumulated. fp32 sums of `rows` terms in any order:
+    rows * 2^-24 of the sum of magnitudes."""
+    s = gpu_scheduler
+    torch.manual_seed(rows + n)
+    st = C.linear_init(s, 8, n, bias=True)
+    x, dy = torch.zeros(rows, 8, device="cuda", dtype=BF), torch.randn(rows, n, device="cuda").to(BF)
+    want, bound = dy.double().sum(0), rows * 2.0 ** -24 * dy.double().abs().sum(0) + 1e-30
+    for step in (1, 2):
+        with cs.autocast(s, BF):
+            C.linear_forward(s, st, T(x))
+        C.linear_backward_parameter(s, st, T(dy))
+        s.synchronize()
+        assert ((st.grad_bias.raw().double() - step * want).abs() <= step * bound).all()
+    assert st.grad_bias.raw().shape == (n,) and st.grad_bias.raw().dtype == torch.float32
