@@ -347,7 +347,6 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
   uint32_t acc[2][32];
   tcgen05_ld_32x32b_x32(taddr, acc[0]);
   float run_max = -INFINITY, run_sum = 0.f;  // base-2 softmax partials
-  uint32_t held[EPI == kEpiGeluDual ? 32 : 1];
   uint32_t box = 0;
 #pragma unroll
   for (int ch = 0; ch < CHUNKS; ++ch) {
@@ -390,31 +389,45 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
             return false;
           }
         }
+        // all loads, all arithmetic, all stores: sixteen independent pairs hide each other's latency
+        uint32_t w[4][4];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint32_t w[4];
-          ld_shared_v4(staging_addr(box, lane, sub * 4 + g), w);
+        for (int g = 0; g < 4; ++g) ld_shared_v4(staging_addr(box, lane, sub * 4 + g), w[g]);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const F2 a = f2_unpack_bf16(w[i]);
-            const F2 x = f2(__uint_as_float(v[g * 8 + 2 * i]), __uint_as_float(v[g * 8 + 2 * i + 1]));
-            float s0, s1;
-            f2_split(EPI == kEpiResidualBf16 ? f2_add(x, a) : f2_mul(x, gelu_grad_pair(a)), s0, s1);
-            w[i] = pack_bf16(s0, s1);
-          }
-          st_shared_v4(staging_addr(box, lane, sub * 4 + g), w[0], w[1], w[2], w[3]);
+        for (int i = 0; i < 16; ++i) {
+          const F2 a = f2_unpack_bf16(w[i >> 2][i & 3]);
+          const F2 x = f2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+          float s0, s1;
+          f2_split(EPI == kEpiResidualBf16 ? f2_add(x, a) : f2_mul(x, gelu_grad_pair(a)), s0, s1);
+          w[i >> 2][i & 3] = pack_bf16(s0, s1);
         }
+#pragma unroll
+        for (int g = 0; g < 4; ++g) st_shared_v4(staging_addr(box, lane, sub * 4 + g), w[g][0], w[g][1], w[g][2], w[g][3]);
       } else {
-        if (sub == 0) box = staging_acquire(st, lane);
-        uint32_t packed[16];
+        uint32_t packed[16], activated[EPI == kEpiGeluDual ? 16 : 1];
 #pragma unroll
         for (int i = 0; i < 16; ++i) packed[i] = pack_bf16(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+        if constexpr (EPI == kEpiGeluDual) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) activated[i] = gelu_pack(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+        }
+        if (sub == 0) {
+          if constexpr (EPI == kEpiGeluDual) {  // both boxes, whose stores have had the time of the arithmetic above
+            if (lane == 0) bulk_wait_read_0();
+            __syncwarp();
+            box = st.base;
+          } else {
+            box = staging_acquire(st, lane);
+          }
+        }
 #pragma unroll
         for (int g = 0; g < 4; ++g)
           st_shared_v4(staging_addr(box, lane, sub * 4 + g), packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]);
         if constexpr (EPI == kEpiGeluDual) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) held[sub * 16 + i] = gelu_pack(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+          for (int g = 0; g < 4; ++g)
+            st_shared_v4(staging_addr(box + EPI_BUF_BYTES, lane, sub * 4 + g), activated[4 * g], activated[4 * g + 1], activated[4 * g + 2],
+                         activated[4 * g + 3]);
         }
         if constexpr (EPI == kEpiCrossEntropy) {
           // running (max, sum-exp) over the valid columns, on the logits as stored (bf16)
@@ -468,12 +481,7 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
         const int c0 = gcol - 32;
         const bool in_range = rows_in_range && c0 < p.n;
         staging_release(map_d, box, c0, row0 - store_row_base, in_range, false, lane);
-        if constexpr (EPI == kEpiGeluDual) {
-          const uint32_t box2 = staging_acquire(st, lane);
-#pragma unroll
-          for (int g = 0; g < 8; ++g) st_shared_v4(staging_addr(box2, lane, g), held[4 * g], held[4 * g + 1], held[4 * g + 2], held[4 * g + 3]);
-          staging_release(map_d2, box2, c0, row0 - store_row_base, in_range, false, lane);
-        }
+        if constexpr (EPI == kEpiGeluDual) staging_release(map_d2, box + EPI_BUF_BYTES, c0, row0 - store_row_base, in_range, false, lane);
       }
     }
   }
