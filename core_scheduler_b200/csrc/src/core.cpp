@@ -3,6 +3,7 @@
 // autocast guard and the blocking to_torch bridge. See cs/core.h for the parity map.
 #include "cs/core.h"
 
+#include <atomic>
 #include <ATen/CPUGeneratorImpl.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAGeneratorImpl.h>
@@ -135,6 +136,10 @@ struct Event::Impl {
   cudaEvent_t ev{nullptr};
   int device{-1};
   bool recorded{false};
+  // Number of records, and the one that a query has found complete: a completed event stays so until it is recorded again,
+  // and asking the driver each time costs about a microsecond per input of a task. A record on another thread between a
+  // query and the note of its result changes `records`, so that the note does not stand for the new record.
+  std::atomic<uint64_t> records{0}, complete{0};
   ~Impl() {
     if (ev) event_pool().release(device, ev);
   }
@@ -158,7 +163,9 @@ void Event::record() const {
     impl_->ev = event_pool().acquire(device);
     impl_->device = device;
   }
+  impl_->records.fetch_add(1, std::memory_order_acq_rel);  // before the record: a query that overlaps must not vouch for it
   CS_CHECK_CUDART(cudaEventRecord(impl_->ev, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream()));
+  impl_->records.fetch_add(1, std::memory_order_acq_rel);
 }
 
 void Event::block() const {
@@ -169,8 +176,13 @@ void Event::block() const {
 
 bool Event::query() const {
   if (!impl_->ev) return true;
+  const uint64_t seen = impl_->records.load(std::memory_order_acquire);
+  if (impl_->complete.load(std::memory_order_acquire) == seen) return true;
   const cudaError_t code = cudaEventQuery(impl_->ev);
-  if (code == cudaSuccess) return true;
+  if (code == cudaSuccess) {
+    if ((seen & 1) == 0) impl_->complete.store(seen, std::memory_order_release);  // odd: a record is under way
+    return true;
+  }
   if (code == cudaErrorNotReady) {
     (void)cudaGetLastError();
     return false;
