@@ -38,7 +38,7 @@ constexpr int TILE_BYTES = 128 * HD * 2;      // 16 KB: a 128-row tile
 constexpr int THREADS = 192;
 constexpr int FWD_CTAS_PER_SM = 2;
 constexpr int FWD_STAGES = 2;
-constexpr int SMEM_BYTES = 2 * TILE_BYTES + FWD_STAGES * 2 * TILE_BYTES + 1024 + 256;  // ~97 KB
+constexpr int SMEM_BYTES = TILE_BYTES + FWD_STAGES * 2 * TILE_BYTES + 1024 + 256;  // ~81 KB
 constexpr int TMEM_COLS = 256;  // S 128, P 64, O 64
 constexpr long long kWaitBudgetCycles = 4000000000LL;
 
@@ -214,48 +214,33 @@ struct AttnParams {
   int causal;           // 1: keys after the query are masked; 0: every query sees every key
 };
 
-// The k-th block of this CTA. Blocks come in order of falling length and are dealt out back and forth, so that no CTA gets
-// the longest one of every round.
-__device__ __forceinline__ int deal(int k) { return k * gridDim.x + ((k & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x); }
-
-// One 128-query block of one head.
-struct FwdItem {
-  int b, h, qb, num_kv;
-};
-__device__ __forceinline__ FwdItem fwd_item(const AttnParams &p, int id) {
-  // every head's longest block of queries first, its shortest last
-  const int heads = p.B * p.H, order = id / heads, bh = id - order * heads;
-  FwdItem it;
-  it.qb = p.T / BQ - 1 - order;
-  it.b = bh / p.H;
-  it.h = bh - it.b * p.H;
-  it.num_kv = p.causal ? it.qb + 1 : p.T / BKV;
-  return it;
-}
-
 __global__ void __launch_bounds__(THREADS, FWD_CTAS_PER_SM) attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv,
                                                                                  const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *aligned = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t q_smem = base;                                    // two buffers of 128 x 64
-  const uint32_t kv_smem = q_smem + 2 * TILE_BYTES;                // per stage: K tile, V tile
+  const uint32_t q_smem = base;                                    // 128 x 64
+  const uint32_t kv_smem = q_smem + TILE_BYTES;                    // per stage: K tile, V tile
   const uint32_t bar_base = kv_smem + FWD_STAGES * 2 * TILE_BYTES;
   uint64_t *bars = reinterpret_cast<uint64_t *>(aligned + (bar_base - base));
-  enum { Q_FULL = 0, Q_EMPTY = 2, S_FULL = 4, S_EMPTY, P_FULL, O_DONE, K_FULL, V_FULL = K_FULL + FWD_STAGES, K_EMPTY = V_FULL + FWD_STAGES,
+  enum { Q_FULL = 0, S_FULL, S_EMPTY, P_FULL, O_DONE, K_FULL, V_FULL = K_FULL + FWD_STAGES, K_EMPTY = V_FULL + FWD_STAGES,
          V_EMPTY = K_EMPTY + FWD_STAGES, NUM_BARS = V_EMPTY + FWD_STAGES };
   auto bar = [&](int i) { return bar_base + 8u * i; };
   volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(bars + NUM_BARS);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + NUM_BARS + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int items = p.B * p.H * (p.T / BQ);
+  // every head's longest block of queries first, its shortest last
+  const int heads = p.B * p.H;
+  const int qb = p.T / BQ - 1 - static_cast<int>(blockIdx.x) / heads;
+  const int bh = static_cast<int>(blockIdx.x) % heads;
+  const int b = bh / p.H, h = bh - b * p.H;
+  const int q0 = qb * BQ;
+  const int num_kv = p.causal ? qb + 1 : p.T / BKV;
+  const int row_base = b * p.T;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(bar(Q_FULL + s), 1);
-      mbar_init(bar(Q_EMPTY + s), 1);
-    }
+    mbar_init(bar(Q_FULL), 1);
     mbar_init(bar(S_FULL), 1);
     mbar_init(bar(S_EMPTY), 4);  // one arrival per softmax warp
     mbar_init(bar(P_FULL), 4);
@@ -284,216 +269,183 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS_PER_SM) attention_fwd_kernel
   const uint32_t o_tmem = p_tmem + BKV / 2;      // 64 columns of output accumulator
 
   if (warp == 0) {
-    int s = 0, qbuf = 0;
-    uint32_t ph = 0, qph = 0;
-    bool ok = true;
-    for (int k = 0, id; ok && (id = deal(k)) < items; ++k) {
-      const FwdItem it = fwd_item(p, id);
-      const int q_col = it.h * HD, k_col = (p.H + it.h) * HD, v_col = (2 * p.H + it.h) * HD, row_base = it.b * p.T;
-      ok = mbar_wait_warp(bar(Q_EMPTY + qbuf), qph ^ 1u, abort_flag);
-      if (!ok) break;
+    const int q_col = h * HD, k_col = (p.H + h) * HD, v_col = (2 * p.H + h) * HD;
+    if (elect_one()) {
+      mbar_expect_tx(bar(Q_FULL), TILE_BYTES);
+      tma_load_2d(q_smem, &map_qkv, bar(Q_FULL), q_col, row_base + q0);
+    }
+    int s = 0;
+    uint32_t ph = 0;
+    for (int j = 0; j < num_kv; ++j) {
+      const uint32_t k_dst = kv_smem + s * 2 * TILE_BYTES;
+      if (!mbar_wait_warp(bar(K_EMPTY + s), ph ^ 1u, abort_flag)) break;
       if (elect_one()) {
-        mbar_expect_tx(bar(Q_FULL + qbuf), TILE_BYTES);
-        tma_load_2d(q_smem + qbuf * TILE_BYTES, &map_qkv, bar(Q_FULL + qbuf), q_col, row_base + it.qb * BQ);
+        mbar_expect_tx(bar(K_FULL + s), TILE_BYTES);
+        tma_load_2d(k_dst, &map_qkv, bar(K_FULL + s), k_col, row_base + j * BKV);
       }
-      qbuf ^= 1;
-      if (qbuf == 0) qph ^= 1u;
-      for (int j = 0; j < it.num_kv; ++j) {
-        const uint32_t k_dst = kv_smem + s * 2 * TILE_BYTES;
-        ok = mbar_wait_warp(bar(K_EMPTY + s), ph ^ 1u, abort_flag);
-        if (!ok) break;
-        if (elect_one()) {
-          mbar_expect_tx(bar(K_FULL + s), TILE_BYTES);
-          tma_load_2d(k_dst, &map_qkv, bar(K_FULL + s), k_col, row_base + j * BKV);
-        }
-        ok = mbar_wait_warp(bar(V_EMPTY + s), ph ^ 1u, abort_flag);
-        if (!ok) break;
-        if (elect_one()) {
-          mbar_expect_tx(bar(V_FULL + s), TILE_BYTES);
-          tma_load_2d(k_dst + TILE_BYTES, &map_qkv, bar(V_FULL + s), v_col, row_base + j * BKV);
-        }
-        if (++s == FWD_STAGES) {
-          s = 0;
-          ph ^= 1u;
-        }
+      if (!mbar_wait_warp(bar(V_EMPTY + s), ph ^ 1u, abort_flag)) break;
+      if (elect_one()) {
+        mbar_expect_tx(bar(V_FULL + s), TILE_BYTES);
+        tma_load_2d(k_dst + TILE_BYTES, &map_qkv, bar(V_FULL + s), v_col, row_base + j * BKV);
+      }
+      if (++s == FWD_STAGES) {
+        s = 0;
+        ph ^= 1u;
       }
     }
   } else if (warp == 1) {
     // S = Q K^T: M=128, N=128, both operands K-major. O += P V: M=128, N=64, A (= P) from TMEM, B (= V) MN-major.
     constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BKV >> 3) << 17) | (8u << 24);
     constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (static_cast<uint32_t>(HD >> 3) << 17) | (8u << 24);
-    // descriptors are built once; a k-step, a stage or a buffer only advances the 16-byte-unit address field
+    // descriptors are built once; a k-step or a stage only advances the 16-byte-unit address field
     const uint64_t d_q = smem_desc(q_smem, 16, 1024), d_k = smem_desc(kv_smem, 16, 1024);
     const uint64_t d_v = smem_desc(kv_smem + TILE_BYTES, 8192, 1024);
-    constexpr uint64_t kStepK = 32 >> 4, kStepMN = 2048 >> 4, kStage = (2 * TILE_BYTES) >> 4, kBuffer = TILE_BYTES >> 4;
-    // the block whose scores are issued next runs one ahead of the accumulating one, across items
-    int f_k = 0, f_id = deal(0), f_j = 0, f_n = f_id < items ? fwd_item(p, f_id).num_kv : 0, f_s = 0, f_buf = 0;
-    uint32_t f_ph = 0, f_qph = 0, f_parity = 0;
-    auto issue_s = [&]() -> bool {  // false: aborted; without work left it does nothing
-      if (f_id >= items) return true;
-      if (f_j == 0 && !mbar_wait_warp(bar(Q_FULL + f_buf), f_qph, abort_flag)) return false;
-      if (!mbar_wait_warp(bar(K_FULL + f_s), f_ph, abort_flag)) return false;
-      if (!mbar_wait_warp(bar(S_EMPTY), f_parity ^ 1u, abort_flag)) return false;  // the softmax warps have read the last S
+    constexpr uint64_t kStepK = 32 >> 4, kStepMN = 2048 >> 4, kStage = (2 * TILE_BYTES) >> 4;
+    bool ok = mbar_wait_warp(bar(Q_FULL), 0, abort_flag);
+    int ks = 0, vs = 0;
+    uint32_t kph = 0, vph = 0;
+    auto issue_s = [&](int j) -> bool {
+      if (!mbar_wait_warp(bar(K_FULL + ks), kph, abort_flag)) return false;
+      if (!mbar_wait_warp(bar(S_EMPTY), (j & 1) ^ 1u, abort_flag)) return false;  // softmax of block j-1 has read S
       fence_after();
-      const uint64_t dq = d_q + f_buf * kBuffer, dk = d_k + f_s * kStage;
-      const bool last = f_j + 1 == f_n;
+      const uint64_t dk = d_k + ks * kStage;
       if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k) umma(s_tmem, dq + k * kStepK, dk + k * kStepK, idesc_s, k > 0 ? 1u : 0u);
+        for (int k = 0; k < HD / 16; ++k) umma(s_tmem, d_q + k * kStepK, dk + k * kStepK, idesc_s, k > 0 ? 1u : 0u);
         umma_commit(bar(S_FULL));
-        umma_commit(bar(K_EMPTY + f_s));
+        umma_commit(bar(K_EMPTY + ks));
       }
-      if (last && elect_one()) umma_commit(bar(Q_EMPTY + f_buf));
-      f_parity ^= 1u;
-      if (++f_s == FWD_STAGES) {
-        f_s = 0;
-        f_ph ^= 1u;
-      }
-      ++f_j;
-      if (last) {
-        f_j = 0;
-        f_buf ^= 1;
-        if (f_buf == 0) f_qph ^= 1u;
-        f_id = deal(++f_k);
-        if (f_id < items) f_n = fwd_item(p, f_id).num_kv;
+      if (++ks == FWD_STAGES) {
+        ks = 0;
+        kph ^= 1u;
       }
       return true;
     };
-    bool ok = issue_s();
-    int s = 0;
-    uint32_t ph = 0, parity = 0;
-    for (int k = 0, id; ok && (id = deal(k)) < items; ++k) {
-      const int num_kv = fwd_item(p, id).num_kv;
-      for (int j = 0; j < num_kv; ++j) {
-        // the next scores are issued as soon as the softmax warps hold this block's
-        ok = issue_s() && mbar_wait_warp(bar(V_FULL + s), ph, abort_flag) && mbar_wait_warp(bar(P_FULL), parity, abort_flag);
-        if (!ok) break;
-        parity ^= 1u;
-        fence_after();
-        const uint64_t dv = d_v + s * kStage;
-        if (elect_one()) {
+    if (ok) ok = issue_s(0);
+    for (int j = 0; ok && j < num_kv; ++j) {
+      if (j + 1 < num_kv) ok = issue_s(j + 1);  // as soon as the softmax warps hold the scores of block j
+      if (!ok) break;
+      if (!mbar_wait_warp(bar(V_FULL + vs), vph, abort_flag)) break;
+      if (!mbar_wait_warp(bar(P_FULL), j & 1, abort_flag)) break;
+      fence_after();
+      const uint64_t dv = d_v + vs * kStage;
+      if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BKV / 16; ++kk)  // 16 keys: 8 columns of P, 2 KB of the MN-major V
-            umma_ts(o_tmem, p_tmem + kk * 8, dv + kk * kStepMN, idesc_o, (j | kk) ? 1u : 0u);
-          umma_commit(bar(O_DONE));
-          umma_commit(bar(V_EMPTY + s));
-        }
-        if (++s == FWD_STAGES) {
-          s = 0;
-          ph ^= 1u;
-        }
+        for (int k = 0; k < BKV / 16; ++k)  // 16 keys: 8 columns of P, 2 KB of the MN-major V
+          umma_ts(o_tmem, p_tmem + k * 8, dv + k * kStepMN, idesc_o, (j | k) ? 1u : 0u);
+        umma_commit(bar(O_DONE));
+        umma_commit(bar(V_EMPTY + vs));
+      }
+      if (++vs == FWD_STAGES) {
+        vs = 0;
+        vph ^= 1u;
       }
     }
   } else {
     const int q = warp & 3;
     const int r = q * 32 + lane;  // query row inside the block
+    const int q_idx = q0 + r;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
-    uint32_t parity = 0;
+    float m_run = -INFINITY, l_run = 0.f;  // m_run: the maximum the exponents refer to (may lag the true one)
     bool ok = true;
-    for (int k = 0, id; ok && (id = deal(k)) < items; ++k) {
-      const FwdItem it = fwd_item(p, id);
-      const int q_idx = it.qb * BQ + r, row_base = it.b * p.T;
-      float m_run = -INFINITY, l_run = 0.f;  // m_run: the maximum the exponents refer to (may lag the true one)
-      for (int j = 0; j < it.num_kv; ++j) {
-        ok = mbar_wait_warp(bar(S_FULL), parity, abort_flag);
-        if (!ok) break;
-        fence_after();
-        uint32_t v[4][32];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32(s_tmem + c * 32 + lane_addr, v[c]);
-        tmem_wait_ld();
-        // the scores sit in registers: the tensor core may start the next block's
-        fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(S_EMPTY));
-        if (p.causal && j == it.qb) {  // the diagonal block: key i of it is visible from row i on
-#pragma unroll
-          for (int c = 0; c < 4; ++c) mask_columns(v[c], ~columns_from(r + 1 - c * 32));
-        }
-        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = fmaxf(fmaxf(mx[(i >> 1) & 3], __uint_as_float(v[c][i])), __uint_as_float(v[c][i + 1]));
-        const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-        // Move the reference maximum only when it lags by more than 2^8 (always on the first block).
-        const bool grow = j == 0 || (m_blk - m_run) * p.scale_log2e > 8.0f;
-        float alpha = 1.0f;
-        if (grow) {
-          alpha = fast_exp2((m_run - m_blk) * p.scale_log2e);  // first block: exp2(-inf) = 0
-          m_run = m_blk;
-          l_run *= alpha;
-        }
-        const float shift = -m_run * p.scale_log2e;
-        const F2 scale2 = f2(p.scale_log2e, p.scale_log2e), shift2 = f2(shift, shift);
-        F2 sum[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
-        uint32_t pk[4][16];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            float a, d;
-            f2_split(f2_fma(f2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), scale2, shift2), a, d);
-            a = fast_exp2(a);
-            d = fast_exp2(d);
-            sum[i & 1] = f2_add(sum[i & 1], f2(a, d));
-            pk[c][i] = pack2(a, d);
-          }
-          if (c == 0 && j > 0) {
-            // P V of block j-1 has read P and completed O before either is touched again
-            ok = mbar_wait_warp(bar(O_DONE), parity ^ 1u, abort_flag);
-            if (!ok) break;
-            fence_after();
-            if (__any_sync(0xffffffffu, grow)) {  // rescale this warp's 32 rows of O in place
-#pragma unroll 1
-              for (int cc = 0; cc < 4; ++cc) {
-                uint32_t ov[16];
-                tmem_ld16(o_tmem + cc * 16 + lane_addr, ov);
-                tmem_wait_ld();
-#pragma unroll
-                for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-                tmem_st16(o_tmem + cc * 16 + lane_addr, ov);
-              }
-            }
-          }
-          tmem_st16(p_tmem + c * 16 + lane_addr, pk[c]);
-        }
-        if (!ok) break;
-        tmem_wait_st();
-        fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(P_FULL));
-        float a, d;
-        f2_split(f2_add(sum[0], sum[1]), a, d);
-        l_run += a + d;
-        parity ^= 1u;
-      }
-      // the last block's P V completes the accumulator
-      ok = ok && mbar_wait_warp(bar(O_DONE), parity ^ 1u, abort_flag);
+    for (int j = 0; j < num_kv; ++j) {
+      const uint32_t ph = j & 1;
+      ok = mbar_wait_warp(bar(S_FULL), ph, abort_flag);
       if (!ok) break;
       fence_after();
+      uint32_t v[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld32(s_tmem + c * 32 + lane_addr, v[c]);
+      tmem_wait_ld();
+      // the scores sit in registers: the tensor core may start the next block's
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(S_EMPTY));
+      if (p.causal && j == qb) {  // the diagonal block: key i of it is visible from row i on
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mask_columns(v[c], ~columns_from(r + 1 - c * 32));
+      }
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = fmaxf(fmaxf(mx[(i >> 1) & 3], __uint_as_float(v[c][i])), __uint_as_float(v[c][i + 1]));
+      const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      // Move the reference maximum only when it lags by more than 2^8 (always on the first block).
+      const bool grow = j == 0 || (m_blk - m_run) * p.scale_log2e > 8.0f;
+      float alpha = 1.0f;
+      if (grow) {
+        alpha = fast_exp2((m_run - m_blk) * p.scale_log2e);  // first block: exp2(-inf) = 0
+        m_run = m_blk;
+        l_run *= alpha;
+      }
+      const float shift = -m_run * p.scale_log2e;
+      const F2 scale2 = f2(p.scale_log2e, p.scale_log2e), shift2 = f2(shift, shift);
+      F2 sum[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
+      uint32_t pk[4][16];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float a, d;
+          f2_split(f2_fma(f2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), scale2, shift2), a, d);
+          a = fast_exp2(a);
+          d = fast_exp2(d);
+          sum[i & 1] = f2_add(sum[i & 1], f2(a, d));
+          pk[c][i] = pack2(a, d);
+        }
+        if (c == 0 && j > 0) {
+          // P V of block j-1 has read P and completed O before either is touched again
+          ok = mbar_wait_warp(bar(O_DONE), ph ^ 1u, abort_flag);
+          if (!ok) break;
+          fence_after();
+          if (__any_sync(0xffffffffu, grow)) {  // rescale this warp's 32 rows of O in place
+#pragma unroll 1
+            for (int cc = 0; cc < 4; ++cc) {
+              uint32_t ov[16];
+              tmem_ld16(o_tmem + cc * 16 + lane_addr, ov);
+              tmem_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+              tmem_st16(o_tmem + cc * 16 + lane_addr, ov);
+            }
+          }
+        }
+        tmem_st16(p_tmem + c * 16 + lane_addr, pk[c]);
+      }
+      if (!ok) break;
+      tmem_wait_st();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(P_FULL));
+      float a, d;
+      f2_split(f2_add(sum[0], sum[1]), a, d);
+      l_run += a + d;
+    }
+    // the last block's P V completes the accumulator
+    const bool done = ok && mbar_wait_warp(bar(O_DONE), (num_kv - 1) & 1, abort_flag);
+    if (done && !*abort_flag && q_idx < p.T &&
+        CS_IN_BOUNDS(kKidAttention, (static_cast<long long>(row_base + q_idx) * p.H + h) * HD + HD - 1,
+                     static_cast<long long>(p.B) * p.T * p.H * HD)) {
+      fence_after();
+      const float inv = 1.f / l_run;
+      __nv_bfloat16 *dst = p.out + (static_cast<long long>(row_base + q_idx) * p.H + h) * HD;
       uint32_t o[2][32];
       tmem_ld32(o_tmem + lane_addr, o[0]);
       tmem_ld32(o_tmem + 32 + lane_addr, o[1]);
       tmem_wait_ld();
-      fence_before();  // the next block's first P_FULL tells the MMA warp that O has been read
-      if (CS_IN_BOUNDS(kKidAttention, (static_cast<long long>(row_base + q_idx) * p.H + it.h) * HD + HD - 1,
-                       static_cast<long long>(p.B) * p.T * p.H * HD)) {
-        const float inv = 1.f / l_run;
-        __nv_bfloat16 *dst = p.out + (static_cast<long long>(row_base + q_idx) * p.H + it.h) * HD;
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const uint32_t(&w8)[32] = o[g >> 2];
-          const int at = (g & 3) * 8;
-          uint4 w;
-          w.x = pack2(__uint_as_float(w8[at + 0]) * inv, __uint_as_float(w8[at + 1]) * inv);
-          w.y = pack2(__uint_as_float(w8[at + 2]) * inv, __uint_as_float(w8[at + 3]) * inv);
-          w.z = pack2(__uint_as_float(w8[at + 4]) * inv, __uint_as_float(w8[at + 5]) * inv);
-          w.w = pack2(__uint_as_float(w8[at + 6]) * inv, __uint_as_float(w8[at + 7]) * inv);
-          *reinterpret_cast<uint4 *>(dst + g * 8) = w;
-        }
-        p.lse[(static_cast<long long>(it.b) * p.H + it.h) * p.T + q_idx] = m_run * p.scale + __logf(l_run);
+      for (int g = 0; g < 8; ++g) {
+        const uint32_t(&w8)[32] = o[g >> 2];
+        const int at = (g & 3) * 8;
+        uint4 w;
+        w.x = pack2(__uint_as_float(w8[at + 0]) * inv, __uint_as_float(w8[at + 1]) * inv);
+        w.y = pack2(__uint_as_float(w8[at + 2]) * inv, __uint_as_float(w8[at + 3]) * inv);
+        w.z = pack2(__uint_as_float(w8[at + 4]) * inv, __uint_as_float(w8[at + 5]) * inv);
+        w.w = pack2(__uint_as_float(w8[at + 6]) * inv, __uint_as_float(w8[at + 7]) * inv);
+        *reinterpret_cast<uint4 *>(dst + g * 8) = w;
       }
+      p.lse[(static_cast<long long>(b) * p.H + h) * p.T + q_idx] = m_run * p.scale + __logf(l_run);
     }
   }
 
@@ -613,6 +565,10 @@ __device__ __forceinline__ BwdItem bwd_item(const AttnBwdParams &p, int id) {
   it.n_iter = kDKV ? 2 * blocks - it.c_first : 2 * (p.causal ? rb + 1 : blocks);
   return it;
 }
+// The k-th block of this CTA. Blocks come in order of falling length and are dealt out back and forth, so that no CTA gets
+// the longest one of every round.
+__device__ __forceinline__ int bwd_deal(int k) { return k * gridDim.x + ((k & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x); }
+
 template <bool kDKV>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_constant__ CUtensorMap qkv_c,
@@ -673,7 +629,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
     int s = 0, rbuf = 0;
     uint32_t ph = 0, rph = 0;
     bool ok = true;
-    for (int k = 0, id; ok && (id = deal(k)) < items; ++k) {
+    for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
       const BwdItem it = bwd_item<kDKV>(p, id);
       const int q_col = it.h * HD, k_col = (p.H + it.h) * HD, v_col = (2 * p.H + it.h) * HD, row_base = it.b * p.T;
       ok = mbar_wait_warp(bar(R_EMPTY + rbuf), rph ^ 1u, abort_flag);
@@ -721,7 +677,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
     int s = 0, g = 0, rbuf = 0;
     uint32_t cph = 0, gph = 0, rph = 0;
     bool ok = true;
-    for (int k = 0, id; ok && (id = deal(k)) < items; ++k) {
+    for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
       const int n_iter = bwd_item<kDKV>(p, id).n_iter;
       ok = mbar_wait_warp(bar(R_FULL + rbuf), rph, abort_flag);
       if (!ok) break;
@@ -761,7 +717,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
     int s = 0, g = 0;
     uint32_t gph = 0, item_parity = 0;
     bool ok = true;
-    for (int k = 0, id; ok && (id = deal(k)) < items; ++k) {
+    for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
       const int n_iter = bwd_item<kDKV>(p, id).n_iter;
       ok = mbar_wait_warp(bar(ACC_EMPTY), item_parity ^ 1u, abort_flag);  // the accumulators of the block before have been read
       item_parity ^= 1u;
@@ -799,7 +755,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
     int s = g;           // stage of that tile
     uint32_t cph = 0, parity = 0;
     bool ok = true;
-    for (int k = 0, id; ok && (id = deal(k)) < items; ++k) {
+    for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
       const BwdItem it = bwd_item<kDKV>(p, id);
       if (next >= it.n_iter) {
         next -= it.n_iter;
@@ -880,7 +836,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
     const int r = q * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     uint32_t parity = 0;
-    for (int k = 0, id; (id = deal(k)) < items; ++k) {
+    for (int k = 0, id; (id = bwd_deal(k)) < items; ++k) {
       const BwdItem it = bwd_item<kDKV>(p, id);
       if (!mbar_wait_warp(bar(ACC_FULL), parity, abort_flag)) break;
       parity ^= 1u;
@@ -978,15 +934,6 @@ bool attn_map(CUtensorMap *out, const void *ptr, int64_t cols, int64_t rows, int
   cache.emplace(key, *out);
   return true;
 }
-int attn_sm_count() {
-  static const int count = [] {
-    int dev = 0, n = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n;
-  }();
-  return count;
-}
 DeviceStatus *attn_status_ptr() {
   static DeviceStatus *ptr = [] {
     void *p = nullptr;
@@ -1018,8 +965,7 @@ int attention_forward_packed(stream_t stream, const void *qkv, void *out, float 
   p.scale_log2e = scale * 1.4426950408889634f;
   p.status = attn_status_ptr();
   p.causal = causal ? 1 : 0;
-  const int64_t items = T / BQ * H * B, most = FWD_CTAS_PER_SM * attn_sm_count();
-  attention_fwd_kernel<<<static_cast<unsigned>(items < most ? items : most), THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(map_qkv, p);
+  attention_fwd_kernel<<<static_cast<unsigned>(T / BQ * H * B), THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(map_qkv, p);
   return finish_launch(1);
 }
 
@@ -1056,7 +1002,13 @@ int attention_backward_packed(stream_t stream, const void *qkv, const void *out,
   p.status = attn_status_ptr();
   p.causal = causal ? 1 : 0;
   const int64_t items = T / 128 * H * B;
-  const auto grid = static_cast<unsigned>(items < attn_sm_count() ? items : attn_sm_count());
+  static const int sm_count = [] {
+    int dev = 0, n = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+  }();
+  const auto grid = static_cast<unsigned>(items < sm_count ? items : sm_count);
   attention_bwd_kernel<true><<<grid, BWD_THREADS, BWD_SMEM_BYTES, s>>>(qkv_r, qkv_c, do_r, do_c, p);
   attention_bwd_kernel<false><<<grid, BWD_THREADS, BWD_SMEM_BYTES, s>>>(qkv_r, qkv_c, do_r, do_c, p);
   return finish_launch(3);
