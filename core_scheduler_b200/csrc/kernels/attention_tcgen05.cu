@@ -1,19 +1,19 @@
 // SPDX-License-Identifier: Apache-2.0
-// Causal self-attention forward on tcgen05 tensor cores for head dimension 64, reading the packed
-// qkv tensor [B, T, 3, H, 64] (the c_attn output) directly and writing [B, T, H*64] plus the
-// per-row log-sum-exp.
+// Self-attention on tcgen05 tensor cores for head dimension 64, causal or not, reading the packed qkv tensor
+// [B, T, 3, H, 64] (the c_attn output) directly. Forward: writes [B, T, H*64] plus the per-row log-sum-exp.
 //
 // One CTA per (batch, head, 128-query block), 192 threads:
-//   warp 0     TMA producer: Q once, then K and V tiles of 64 keys (one stage each)
-//   warp 1     MMA issuer: S = Q K^T (128x64x64, fp32 in TMEM) and
-//              O += P V (128x64x64; P from shared memory, V as an MN-major operand)
-//   warps 2-5  softmax: one thread per query row reads its S row from TMEM, keeps the reference
-//              max / running sum and writes P (bf16, 128-byte swizzled) to shared memory for the
-//              second MMA. O accumulates in TMEM across key blocks; a warp rescales its 32 rows of
-//              O in place only when a row maximum has grown by more than 2^8 since the reference
-//              was taken (probabilities stay below 256, exact after the final division)
-// Four CTAs share an SM (49 KB of shared memory, 128 TMEM columns and at most 85 registers per
-// thread each): sixteen softmax warps per SM hide each other's TMEM, exp and barrier latencies. Scores never touch global memory. Every mbarrier wait is bounded (abort flag + status word).
+//   warp 0     TMA producer: Q once, then K and V tiles of 128 keys (two stages)
+//   warp 1     MMA issuer: S = Q K^T (128x128x64, fp32 in TMEM) and O += P V (128x64x128; P is a bf16 A operand in
+//              TMEM, V an MN-major operand). The scores of block j+1 are issued as soon as those of block j sit in registers
+//   warps 2-5  softmax: one thread per query row reads its row of S once (128 registers), keeps the reference max /
+//              running sum, exponentiates on packed pairs and writes P back to TMEM. O accumulates in TMEM across key
+//              blocks; a warp rescales its 32 rows of O in place only when a row maximum has grown by more than 2^8 since
+//              the reference was taken (probabilities stay below 256, exact after the final division)
+// Two CTAs share an SM (81 KB of shared memory, 256 TMEM columns, 168 registers a thread): one's barriers and loads hide
+// behind the other's exponentials, 1024 cycles a block and what bounds it. 16 x 1024 tokens, 12 heads, causal: 102 -> 58 us
+// against four CTAs with 64-key blocks that read S twice and passed P through shared memory; 2 x 4096, 20 heads
+// 289 -> 122. Scores never touch global memory. Every mbarrier wait is bounded (abort flag + status word).
 //
 // What it replaces in the reference project: at::_scaled_dot_product_flash_attention
 // (src/compute/sdpa_flash_attn.cpp:56-60) and the cuDNN-frontend SDPA graph

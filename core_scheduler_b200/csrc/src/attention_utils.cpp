@@ -81,7 +81,7 @@ bool use_cudnn_engine() {
 }
 
 // This library's own forward and backward kernels on the packed qkv tensor are the default for
-// the shapes they cover (bf16, causal, head dimension 64, T % 128 == 0, no dropout);
+// the shapes they cover (bf16, causal or not, head dimension 64, T % 128 == 0, no dropout);
 // CS_ATTENTION_ENGINE=cudnn or =flash selects a library engine instead. Read at every call (a
 // dozen per step) so that a process can switch engines between models.
 bool use_own_forward() {
