@@ -92,6 +92,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
+// After an abandoned wait: copies into this block's shared memory may still be in flight. Gives them a bounded time to land
+// before the block goes away.
+__device__ __forceinline__ void abort_grace(volatile int *abort_flag) {
+  if (!*abort_flag) return;
+  const long long t0 = clock64();
+  while (clock64() - t0 < 2000000LL) __nanosleep(1000);
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -449,6 +456,7 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS_PER_SM) attention_fwd_kernel
     }
   }
 
+  abort_grace(abort_flag);
   fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag) {
@@ -872,6 +880,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
     }
   }
 
+  abort_grace(abort_flag);
   fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag) {
