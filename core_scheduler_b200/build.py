@@ -197,7 +197,7 @@ def build_examples() -> list[str]:
 
 
 def build_cpp_tests() -> list[str]:
-    """Compiles the C++ test programs under tests/cpp/ (cs_b200_tests, cs_b200_communication_tests) into tests/cpp/bin/."""
+    """Compiles the C++ test programs under tests/cpp/ (cs_b200_tests, cs_b200_communication_tests, test_tensor_map) into tests/cpp/bin/."""
     root = HERE.parent / "tests" / "cpp"
     return _build_programs(root, [root], {"test_ops": "cs_b200_tests", "test_communication": "cs_b200_communication_tests"})
 
@@ -227,7 +227,7 @@ def _build_programs(root: Path, extra_inc: list, names: dict | None = None) -> l
         # up to date = same program source and same headers as when it was compiled (content, not time stamps, which
         # a copy of the tree does not keep); the library itself is linked dynamically
         stamp = out_dir / (exe.name + ".stamp")
-        digest = _sources_digest([src, *root.glob("*.h"), *(f for f in (CSRC / "include").rglob("*.h"))])
+        digest = _sources_digest([src, *root.glob("*.h"), *(CSRC / "include").rglob("*.h"), *(CSRC / "kernels").glob("*.h")])
         if exe.exists() and stamp.exists() and stamp.read_text() == digest:
             built.append(str(exe))
             continue

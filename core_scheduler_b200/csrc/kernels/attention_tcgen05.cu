@@ -23,11 +23,10 @@
 #include <cuda_runtime.h>
 
 #include <cstdlib>
-#include <mutex>
-#include <unordered_map>
 
 #include "api.h"
 #include "bounds_check.h"
+#include "tensor_map.h"
 
 namespace cs::kernels {
 namespace {
@@ -895,22 +894,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
   }
 }
 
-using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                              const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeFn attn_encode_fn() {
-  static EncodeFn fn = [] {
-    void *ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess) {
-      (void)cudaGetLastError();
-      return static_cast<EncodeFn>(nullptr);
-    }
-    return reinterpret_cast<EncodeFn>(ptr);
-  }();
-  return fn;
-}
 }  // namespace
 
 int attention_status(DeviceStatus *out) {
@@ -918,30 +901,10 @@ int attention_status(DeviceStatus *out) {
 }
 
 namespace {
-// [rows, cols] bf16 row-major viewed through 64-column boxes of `box_rows` rows, 128-byte swizzle.
+// [rows, cols] bf16 row-major viewed through 64-column boxes of `box_rows` rows.
 bool attn_map(CUtensorMap *out, const void *ptr, int64_t cols, int64_t rows, int box_rows) {
-  EncodeFn fn = attn_encode_fn();
-  if (!fn) return false;
-  static std::mutex mu;
-  static std::unordered_map<uint64_t, CUtensorMap> cache;
-  std::lock_guard<std::mutex> lock{mu};
-  const uint64_t key = reinterpret_cast<uint64_t>(ptr) ^ (static_cast<uint64_t>(rows) << 40) ^ (static_cast<uint64_t>(cols) << 20) ^
-                       (static_cast<uint64_t>(box_rows) << 56);
-  auto it = cache.find(key);
-  if (it != cache.end()) {
-    *out = it->second;
-    return true;
-  }
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols * 2)};
-  const cuuint32_t box[2] = {HD, static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t elem[2] = {1, 1};
-  if (fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return false;
-  if (cache.size() > 4096) cache.clear();
-  cache.emplace(key, *out);
-  return true;
+  return get_tensor_map(ptr, static_cast<uint64_t>(cols), static_cast<uint64_t>(rows), static_cast<uint64_t>(cols), HD,
+                        static_cast<uint32_t>(box_rows), out);
 }
 DeviceStatus *attn_status_ptr() {
   static DeviceStatus *ptr = [] {

@@ -29,12 +29,11 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
-#include <unordered_map>
 
 #include "api.h"
 #include "bounds_check.h"
 #include "collectives.h"
+#include "tensor_map.h"
 
 namespace cs::kernels {
 namespace {
@@ -871,78 +870,24 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   }
 }
 
-// ------------------------------------------------------------------ host: tensor maps ----
-using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                              const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+}  // namespace
 
-EncodeFn encode_fn() {
-  static EncodeFn fn = [] {
-    void *ptr = nullptr;
+// ------------------------------------------------------------------ host: tensor maps ----
+bool get_tensor_map(const void *ptr, uint64_t inner, uint64_t outer, uint64_t stride_elems, uint32_t box_inner,
+                    uint32_t box_outer, CUtensorMap *out, int elem_bytes) {
+  static const TensorMapEncodeFn encode = [] {
+    void *fn = nullptr;
     cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
         qres != cudaDriverEntryPointSuccess) {
       (void)cudaGetLastError();
-      return static_cast<EncodeFn>(nullptr);
+      return static_cast<TensorMapEncodeFn>(nullptr);
     }
-    return reinterpret_cast<EncodeFn>(ptr);
+    return reinterpret_cast<TensorMapEncodeFn>(fn);
   }();
-  return fn;
+  static TensorMapCache cache;
+  return cache.get(encode, TensorMapKey{ptr, inner, outer, stride_elems * elem_bytes, box_inner, box_outer, elem_bytes}, out);
 }
-
-struct MapKey {
-  const void *ptr;
-  uint64_t inner, outer, stride_bytes;
-  uint32_t box_inner, box_outer;
-  int elem_bytes;
-  bool operator==(const MapKey &o) const {
-    return ptr == o.ptr && inner == o.inner && outer == o.outer && stride_bytes == o.stride_bytes &&
-           box_inner == o.box_inner && box_outer == o.box_outer && elem_bytes == o.elem_bytes;
-  }
-};
-struct MapKeyHash {
-  size_t operator()(const MapKey &k) const {
-    size_t h = reinterpret_cast<size_t>(k.ptr);
-    auto mix = [&h](uint64_t v) { h ^= v + 0x9e3779b97f4a7c15ULL + (h << 6) + (h >> 2); };
-    mix(k.inner);
-    mix(k.outer);
-    mix(k.stride_bytes);
-    mix((static_cast<uint64_t>(k.box_inner) << 32) | k.box_outer);
-    return h;
-  }
-};
-
-// 2-D bf16 tensor map: `inner` contiguous elements per row, `outer` rows, row stride in
-// elements; box = box_inner x box_outer with the 128-byte swizzle (box_inner == 64).
-bool get_tensor_map(const void *ptr, uint64_t inner, uint64_t outer, uint64_t stride_elems, uint32_t box_inner,
-                    uint32_t box_outer, CUtensorMap *out, int elem_bytes = 2) {
-  static std::mutex mu;
-  static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-  const MapKey key{ptr, inner, outer, stride_elems * elem_bytes, box_inner, box_outer, elem_bytes};
-  std::lock_guard<std::mutex> lock{mu};
-  auto it = cache.find(key);
-  if (it != cache.end()) {
-    *out = it->second;
-    return true;
-  }
-  EncodeFn fn = encode_fn();
-  if (!fn) return false;
-  const cuuint64_t dims[2] = {inner, outer};
-  const cuuint64_t strides[1] = {stride_elems * elem_bytes};
-  const cuuint32_t box[2] = {box_inner, box_outer};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  CUtensorMap map;
-  const CUresult r = fn(&map, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, elem_strides,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return false;
-  if (cache.size() > 8192) cache.clear();
-  cache.emplace(key, map);
-  *out = map;
-  return true;
-}
-
-}  // namespace
 
 namespace {
 // Row tiles walked together (group_m): the pairs in flight then cover a block of group_m x (pairs / group_m) tiles, and a
