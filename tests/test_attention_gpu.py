@@ -154,3 +154,43 @@ def test_blocks_dealt_to_persistent_ctas(B, T, H, causal):
     got, want = dqkv.double().view(B, T, 3, H, D), qr.grad.view(B, T, 3, H, D)
     for i in range(3):
         assert ((got[:, :, i] - want[:, :, i]).norm() / want[:, :, i].norm()).item() < 1e-2
+
+
+@pytest.mark.parametrize("row", [0, 37, 63, 64, 127, 190])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+def test_a_query_that_is_not_finite_stays_with_the_keys_it_sees(row, value):
+    """Causal backward with one query row whose log-sum-exp is NaN or infinite: the keys after it get the same bits as without
+    it, in dV and in dK, and no other query's dQ changes."""
+    B, T, H, D = 1, 256, 2, 64
+    torch.manual_seed(row)
+    qkv, dout = torch.randn(B, T, 3 * H * D, device="cuda").to(BF), torch.randn(B, T, H * D, device="cuda").to(BF)
+    rc, out, lse = C.attention_forward_tcgen05(qkv, H, 0.125, causal=True)
+    assert rc == 0
+    clean, _ = C.attention_backward_tcgen05(qkv, out, dout, lse, H, 0.125, causal=True)
+    bad_lse = lse.clone()
+    bad_lse[0, 1, row] = value
+    got, _ = C.attention_backward_tcgen05(qkv, out, dout, bad_lse, H, 0.125, causal=True)
+    clean, got = clean.view(T, 3, H, D), got.view(T, 3, H, D)
+    assert torch.equal(got[:, :, 0], clean[:, :, 0])  # the other head
+    assert torch.equal(got[row + 1:, 1:, 1], clean[row + 1:, 1:, 1])
+    others = torch.arange(T, device="cuda") != row
+    assert torch.equal(got[others, 0, 1], clean[others, 0, 1])
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("scale", [0.125, 0.0, -0.125])
+def test_backward_of_a_given_forward_takes_any_scale(scale, causal):
+    """dqkv from an output and a log-sum-exp computed elsewhere. bf16 P, dS and results: below 1e-2 in the 2-norm."""
+    B, T, H, D = 2, 256, 3, 64
+    torch.manual_seed(5)
+    qkv, dout = torch.randn(B, T, 3 * H * D, device="cuda").to(BF), torch.randn(B, T, H * D, device="cuda").to(BF)
+    qr = qkv.double().requires_grad_(True)
+    q, k, v = (x.transpose(1, 2) for x in qr.view(B, T, 3, H, D).unbind(2))
+    s = q @ k.transpose(2, 3) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(T, T, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    ref = (s.softmax(-1) @ v).transpose(1, 2).reshape(B, T, H * D)
+    ref.backward(dout.double())
+    lse = s.detach().logsumexp(-1).float().contiguous()
+    got, _ = C.attention_backward_tcgen05(qkv, ref.detach().to(BF), dout, lse, H, scale, causal=causal)
+    assert ((got.double() - qr.grad).norm() / qr.grad.norm()).item() < 1e-2
