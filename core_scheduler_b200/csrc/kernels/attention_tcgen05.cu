@@ -22,6 +22,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cfloat>
+#include <cmath>
 #include <cstdlib>
 
 #include "api.h"
@@ -229,6 +231,7 @@ struct AttnParams {
   float scale;
   DeviceStatus *status;
   int causal;           // 1: keys after the query are masked; 0: every query sees every key
+  int negate;           // 1: the tensor core forms -Q K^T, and `scale` is the magnitude of a negative softmax scale
 };
 
 __global__ void __launch_bounds__(THREADS, FWD_CTAS_PER_SM) attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv,
@@ -312,7 +315,7 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS_PER_SM) attention_fwd_kernel
     }
   } else if (warp == 1) {
     // S = Q K^T: M=128, N=128, both operands K-major. O += P V: M=128, N=64, A (= P) from TMEM, B (= V) MN-major.
-    constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BKV >> 3) << 17) | (8u << 24);
+    const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (p.negate ? 1u << 13 : 0u) | (static_cast<uint32_t>(BKV >> 3) << 17) | (8u << 24);
     constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (static_cast<uint32_t>(HD >> 3) << 17) | (8u << 24);
     // descriptors are built once; a k-step or a stage only advances the 16-byte-unit address field
     const uint64_t d_q = smem_desc(q_smem, 16, 1024), d_k = smem_desc(kv_smem, 16, 1024);
@@ -946,8 +949,12 @@ int attention_forward_packed(stream_t stream, const void *qkv, void *out, float 
   p.B = static_cast<int>(B);
   p.T = static_cast<int>(T);
   p.H = static_cast<int>(H);
-  p.scale = scale;
-  p.scale_log2e = scale * 1.4426950408889634f;
+  // The kernel's maximum, its -inf for masked keys and the lag of its reference want a positive scale: a negative one is its
+  // magnitude with the products negated, and zero the smallest normal number, which leaves every finite score at exp(0).
+  const float magnitude = std::fabs(scale);
+  p.negate = scale < 0.f ? 1 : 0;
+  p.scale = magnitude < FLT_MIN ? FLT_MIN : magnitude;
+  p.scale_log2e = p.scale * 1.4426950408889634f;
   p.status = attn_status_ptr();
   p.causal = causal ? 1 : 0;
   attention_fwd_kernel<<<static_cast<unsigned>(T / BQ * H * B), THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(map_qkv, p);
