@@ -361,3 +361,18 @@ def test_bias_gradient_column_sums(gpu_scheduler, rows, n):
         s.synchronize()
         assert ((st.grad_bias.raw().double() - step * want).abs() <= step * bound).all()
     assert st.grad_bias.raw().shape == (n,) and st.grad_bias.raw().dtype == torch.float32
+
+
+@pytest.mark.parametrize("d", [8, 56, 88, 768, 896, 1000, 1792, 2048, 2304])
+def test_layernorm_of_constant_rows_is_the_bias(gpu_scheduler, d):
+    """Rows of one value: their sum is exact in fp32 (8 + 12 bits), so the mean is the value, the deviation zero, and the result
+    the bias to the last bit, however far rstd magnifies."""
+    s = gpu_scheduler
+    st = C.layer_norm_init(s, [d])
+    st.weight.raw().uniform_(0.5, 1.5)
+    st.bias.raw().uniform_(-0.5, 0.5)
+    x = torch.tensor([100.5, -0.0302734375, 3.015625, 1e4, -7.0], device="cuda").to(BF)[:, None].expand(5, d).contiguous()
+    with cs.autocast(s, BF):
+        y = C.layer_norm_forward(s, st, T(x))
+    s.synchronize()
+    assert torch.equal(y.raw(), st.bias.raw().to(BF).expand(5, d))
