@@ -406,12 +406,13 @@ constexpr int kLnWarps = 4;       // rows per CTA iteration
 constexpr int kLnRows = 4;        // rows a CTA of the column kernels has in flight
 constexpr int kLnBwdCtas = kSmCount * 6;
 
-// Rows wider than 2048: one warp per row, grid-stride over rows. Lane l owns the 8-element chunks l, l+32, ... of the
-// row. The next row (still packed, in its 128-bit load registers) is fetched before the current
+// Rows up to 768 columns and wider than 2048: one warp per row, grid-stride over rows. Lane l owns the 8-element chunks
+// l, l+32, ... of the row. The next row (still packed, in its 128-bit load registers) is fetched before the current
 // one is reduced, so that loads stay in flight during the shuffles; the grid is one resident wave.
+constexpr int ln_row_ctas_per_sm(int chunks) { return chunks <= 3 ? 4 : 2; }
 template <int CHUNKS>
-__global__ void __launch_bounds__(kLnWarps * 32, 1)
-ln_fwd_wide_kernel(const __nv_bfloat16 *__restrict__ x, const void *__restrict__ gamma, const void *__restrict__ beta, int pdt,
+__global__ void __launch_bounds__(kLnWarps * 32, CHUNKS <= 3 ? 4 : 1)
+ln_fwd_row_kernel(const __nv_bfloat16 *__restrict__ x, const void *__restrict__ gamma, const void *__restrict__ beta, int pdt,
               __nv_bfloat16 *__restrict__ y, float *__restrict__ mean, float *__restrict__ rstd, int64_t rows, int d, float eps) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nchunks = d / 8;
@@ -426,6 +427,20 @@ ln_fwd_wide_kernel(const __nv_bfloat16 *__restrict__ x, const void *__restrict__
         dst[c] = *reinterpret_cast<const Bf16x8 *>(x + r * d + chunk * 8);
     }
   };
+  // gamma and beta of this lane's chunks stay in registers for narrow rows (they would otherwise be
+  // re-read from L1 for every row: four times the bytes of the row itself)
+  constexpr bool kHoist = CHUNKS <= 3;
+  float gw[kHoist ? CHUNKS : 1][8] = {}, bw[kHoist ? CHUNKS : 1][8] = {};
+  if (kHoist) {
+#pragma unroll
+    for (int c = 0; c < (kHoist ? CHUNKS : 1); ++c) {
+      const int chunk = lane + 32 * c;
+      if (chunk < nchunks) {
+        load8(gamma, chunk * 8, pdt, gw[c]);
+        if (beta) load8(beta, chunk * 8, pdt, bw[c]);
+      }
+    }
+  }
   if (row < rows) load_row(cur, row);
   while (row < rows) {
     const int64_t next = row + stride;
@@ -462,12 +477,20 @@ ln_fwd_wide_kernel(const __nv_bfloat16 *__restrict__ x, const void *__restrict__
       const int chunk = lane + 32 * c;
       if (chunk < nchunks) {
         float g[8], b[8], o[8];
-        load8(gamma, chunk * 8, pdt, g);
-        if (beta) {
-          load8(beta, chunk * 8, pdt, b);
-        } else {
+        if (kHoist) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) b[k] = 0.f;
+          for (int k = 0; k < 8; ++k) {
+            g[k] = gw[kHoist ? c : 0][k];
+            b[k] = bw[kHoist ? c : 0][k];
+          }
+        } else {
+          load8(gamma, chunk * 8, pdt, g);
+          if (beta) {
+            load8(beta, chunk * 8, pdt, b);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) b[k] = 0.f;
+          }
         }
 #pragma unroll
         for (int k = 0; k < 8; ++k) o[k] = (v[c][k] - mu) * rs * g[k] + b[k];
@@ -480,7 +503,7 @@ ln_fwd_wide_kernel(const __nv_bfloat16 *__restrict__ x, const void *__restrict__
   }
 }
 
-// Rows up to 2048 columns: thread t of a CTA owns columns 8t .. 8t+7 and the CTA takes kLnRows rows at a time. gamma, beta
+// Rows up to 2048 columns (forward: from 776 on): thread t of a CTA owns columns 8t .. 8t+7 and the CTA takes kLnRows rows at a time. gamma, beta
 // and the dgamma/dbeta partials of eight columns are 16 to 32 registers, whatever the width, where a warp per row keeps
 // 2 x 8 partials for each of its d / 256 chunks (167 registers, 12 warps an SM) or re-reads gamma and beta from L1 for every
 // row. What a row costs instead is a sum over the CTA's warps: kLnRows of them share one halving butterfly, one barrier and
@@ -725,12 +748,12 @@ int launch_ln_bwd(cudaStream_t s, const void *dy, const void *x, const void *gam
 }
 
 template <int CHUNKS>
-int launch_ln_fwd_wide(cudaStream_t s, const void *x, const void *gamma, const void *beta, int pdt, void *y, float *mean,
+int launch_ln_fwd_rows(cudaStream_t s, const void *x, const void *gamma, const void *beta, int pdt, void *y, float *mean,
                        float *rstd, int64_t rows, int d, float eps) {
   const int64_t blocks = (rows + kLnWarps - 1) / kLnWarps;
-  const int64_t wave = static_cast<int64_t>(kSmCount) * 2;
+  const int64_t wave = static_cast<int64_t>(kSmCount) * ln_row_ctas_per_sm(CHUNKS);
   const int grid = static_cast<int>(blocks > wave ? wave : blocks);
-  ln_fwd_wide_kernel<CHUNKS><<<grid, kLnWarps * 32, 0, s>>>(static_cast<const __nv_bfloat16 *>(x), gamma, beta, pdt,
+  ln_fwd_row_kernel<CHUNKS><<<grid, kLnWarps * 32, 0, s>>>(static_cast<const __nv_bfloat16 *>(x), gamma, beta, pdt,
                                                             static_cast<__nv_bfloat16 *>(y), mean, rstd, rows, d, eps);
   return finish_launch();
 }
@@ -742,8 +765,12 @@ int layernorm_forward(stream_t stream, const void *x, const void *gamma, const v
   if (d % 8 != 0 || d > 8192 || rows == 0) return rows == 0 ? 0 : static_cast<int>(cudaErrorInvalidValue);
   const int chunks = static_cast<int>((d / 8 + 31) / 32);
   const int di = static_cast<int>(d);
-  if (chunks > 16) return launch_ln_fwd_wide<32>(s, x, gamma, beta, param_dtype, y, mean, rstd, rows, di, eps);
-  if (chunks > 8) return launch_ln_fwd_wide<16>(s, x, gamma, beta, param_dtype, y, mean, rstd, rows, di, eps);
+  // The column kernel is the faster one above 768 columns (32768 x 1024: 35 against 39 us, 64 x 1024: 3.5 against 4.2), a warp per
+  // row up to there (32768 x 768: 22 against 31, 32768 x 256: 13 against 21, 64 x 256: 2.7 against 3.5; all from cold caches).
+  if (chunks <= 2) return launch_ln_fwd_rows<2>(s, x, gamma, beta, param_dtype, y, mean, rstd, rows, di, eps);
+  if (chunks <= 3) return launch_ln_fwd_rows<3>(s, x, gamma, beta, param_dtype, y, mean, rstd, rows, di, eps);
+  if (chunks > 16) return launch_ln_fwd_rows<32>(s, x, gamma, beta, param_dtype, y, mean, rstd, rows, di, eps);
+  if (chunks > 8) return launch_ln_fwd_rows<16>(s, x, gamma, beta, param_dtype, y, mean, rstd, rows, di, eps);
   ln_fwd_kernel<<<static_cast<int>(ln_grid(rows, di, 1024, rows)), ln_threads(di), 0, s>>>(
       static_cast<const __nv_bfloat16 *>(x), gamma, beta, param_dtype, static_cast<__nv_bfloat16 *>(y), mean, rstd, rows, di, eps);
   return finish_launch();

@@ -376,3 +376,10 @@ def test_layernorm_of_constant_rows_is_the_bias(gpu_scheduler, d):
         y = C.layer_norm_forward(s, st, T(x))
     s.synchronize()
     assert torch.equal(y.raw(), st.bias.raw().to(BF).expand(5, d))
+
+
+@pytest.mark.parametrize("rows,d", [(1, 768), (3, 776), (2, 512), (5, 584), (7, 592), (4737, 256), (9999, 768), (2961, 776), (1300, 520)])
+def test_layernorm_where_its_dispatch_changes(gpu_scheduler, rows, d):
+    """Around 768 columns (a warp or a CTA per row forward), 592 (columns per block of the gradient sum) and a multiple of 256,
+    with odd row counts below and above one wave of CTAs: the bounds of the test above."""
+    test_layernorm_column_kernels(gpu_scheduler, rows, d)
