@@ -58,9 +58,9 @@ int pack_qkv(stream_t stream, const void *q, const void *k, const void *v, void 
 int layernorm_forward(stream_t stream, const void *x, const void *gamma, const void *beta, int param_dtype, void *y,
                       float *mean, float *rstd, int64_t rows, int64_t d, float eps);
 // Single pass: dx (+ grad_residual when given) and per-CTA partial dgamma/dbeta reduced by a
-// second tiny kernel. `scratch` holds 2 * layernorm_backward_scratch_rows() * d floats.
+// second tiny kernel. `scratch` holds 2 * layernorm_backward_scratch_rows(d) * d floats.
 // dgamma/dbeta are fp32; accumulate != 0 adds to their current contents.
-int64_t layernorm_backward_scratch_rows();
+int64_t layernorm_backward_scratch_rows(int64_t d);
 int layernorm_backward(stream_t stream, const void *dy, const void *x, const void *gamma, int param_dtype,
                        const float *mean, const float *rstd, const void *grad_residual, void *dx, float *dgamma,
                        float *dbeta, int accumulate, float *scratch, int64_t rows, int64_t d);

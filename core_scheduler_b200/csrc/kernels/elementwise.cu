@@ -403,8 +403,8 @@ int pack_qkv(stream_t stream, const void *q, const void *k, const void *v, void 
 // --------------------------------------------------------------------------- LayerNorm ----
 namespace {
 constexpr int kLnWarps = 4;       // rows per CTA iteration
-constexpr int kLnRows = 4;        // rows a CTA of the column kernels has in flight
-constexpr int kLnBwdCtas = kSmCount * 6;
+constexpr int kLnRows = 4;        // rows a CTA of the forward column kernel has in flight
+constexpr int kLnBwdRows = 2;     // rows a CTA of the backward kernel works on, with as many more on their way
 
 // Rows up to 768 columns and wider than 2048: one warp per row, grid-stride over rows. Lane l owns the 8-element chunks
 // l, l+32, ... of the row. The next row (still packed, in its 128-bit load registers) is fetched before the current
@@ -503,12 +503,15 @@ ln_fwd_row_kernel(const __nv_bfloat16 *__restrict__ x, const void *__restrict__ 
   }
 }
 
-// Rows up to 2048 columns (forward: from 776 on): thread t of a CTA owns columns 8t .. 8t+7 and the CTA takes kLnRows rows at a time. gamma, beta
-// and the dgamma/dbeta partials of eight columns are 16 to 32 registers, whatever the width, where a warp per row keeps
-// 2 x 8 partials for each of its d / 256 chunks (167 registers, 12 warps an SM) or re-reads gamma and beta from L1 for every
-// row. What a row costs instead is a sum over the CTA's warps: kLnRows of them share one halving butterfly, one barrier and
-// 512 bytes of shared memory, little enough for a CTA to run beside a resident GEMM block. Bound by HBM: 32768 rows of 1280,
-// forward 50 -> 42 us, backward with the residual gradient 122 -> 84 (four bf16 tensors, 51 at the copy rate).
+// Rows up to 2048 columns (forward: from 776 on): thread t of a CTA owns columns 8t .. 8t+7 and the CTA takes a group of rows at
+// a time. gamma, beta and the dgamma/dbeta partials of eight columns are 16 to 32 registers, whatever the width, where a warp per
+// row keeps 2 x 8 partials for each of its d / 256 chunks (167 registers, 12 warps an SM) or re-reads gamma and beta from L1 for
+// every row. What a row costs instead is a sum over the CTA's warps: the rows of a group share one halving butterfly, one barrier
+// and 256 bytes of shared memory, little enough for a CTA to run beside a resident GEMM block. Forward takes four rows at a time;
+// backward two, with the next two on their way while these meet: four without that left no load in flight between the barriers
+// and was slower than a warp per row below 1000 columns. Bound by HBM, from cold caches, against a warp per row: 32768 x 1280
+// forward 48 -> 44 us, backward with the residual gradient 116 -> 73 (four bf16 tensors, 51 at the copy rate); backward of
+// 32768 x 768 49 -> 46, of 32768 x 256 24 -> 17, of 1024 x 768 7.6 -> 5.0.
 
 // Sums each of N values over the warp; afterwards lane l holds the sum of value l / (32 / N). N shuffles in all but the last
 // rounds instead of N in each of the five.
@@ -613,7 +616,7 @@ __global__ void __launch_bounds__(256, 2) ln_bwd_kernel(const __nv_bfloat16 *__r
                                                      const void *__restrict__ gamma, int pdt, const float *__restrict__ mean,
                                                      const float *__restrict__ rstd, const __nv_bfloat16 *__restrict__ dres,
                                                      __nv_bfloat16 *__restrict__ dx, float *__restrict__ scratch, int64_t rows, int d) {
-  __shared__ float red[2][8][2 * kLnRows];
+  __shared__ float red[2][8][2 * kLnBwdRows];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int col = threadIdx.x * 8;
   const bool active = col < d;
@@ -622,42 +625,71 @@ __global__ void __launch_bounds__(256, 2) ln_bwd_kernel(const __nv_bfloat16 *__r
   for (int k = 0; k < 8; ++k) g[k] = dg[k] = db[k] = 0.f;
   if (active) load8(gamma, col, pdt, g);
   const float inv_d = 1.f / d;
-  const int64_t step = static_cast<int64_t>(gridDim.x) * kLnRows;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kLnBwdRows;
   int buffer = 0;
-  for (int64_t row0 = static_cast<int64_t>(blockIdx.x) * kLnRows; row0 < rows; row0 += step, buffer ^= 1) {
-    Bf16x8 xp[kLnRows] = {}, dp[kLnRows] = {}, rp[kLnRows] = {};
-    float mu[kLnRows], rs[kLnRows], s[2 * kLnRows];
+  // The next rows are on their way while the sums of the present ones meet.
+  Bf16x8 xn[kLnBwdRows] = {}, dn[kLnBwdRows] = {}, rn[kLnBwdRows] = {};
+  float mun[kLnBwdRows], rsn[kLnBwdRows];
+  auto load = [&](int64_t first) {
 #pragma unroll
-    for (int r = 0; r < kLnRows; ++r) {
-      const int64_t row = row0 + r;
+    for (int r = 0; r < kLnBwdRows; ++r) {
+      const int64_t row = first + r;
       const bool in = row < rows;
       if (in && active && CS_IN_BOUNDS(kKidLayerNormBwd, row * d + col + 7, rows * d)) {
-        xp[r] = *reinterpret_cast<const Bf16x8 *>(x + row * d + col);
-        dp[r] = *reinterpret_cast<const Bf16x8 *>(dy + row * d + col);
-        if (dres) rp[r] = *reinterpret_cast<const Bf16x8 *>(dres + row * d + col);
+        xn[r] = *reinterpret_cast<const Bf16x8 *>(x + row * d + col);
+        dn[r] = *reinterpret_cast<const Bf16x8 *>(dy + row * d + col);
+        if (dres) rn[r] = *reinterpret_cast<const Bf16x8 *>(dres + row * d + col);
+      } else {
+        xn[r] = dn[r] = rn[r] = Bf16x8{};
       }
-      mu[r] = in ? mean[row] : 0.f;
-      rs[r] = in ? rstd[row] : 0.f;
+      mun[r] = in ? mean[row] : 0.f;
+      rsn[r] = in ? rstd[row] : 0.f;
     }
+  };
+  int64_t row0 = static_cast<int64_t>(blockIdx.x) * kLnBwdRows;
+  load(row0);
+  for (; row0 < rows; row0 += step, buffer ^= 1) {
+    Bf16x8 xp[kLnBwdRows], dp[kLnBwdRows], rp[kLnBwdRows];
+    float mu[kLnBwdRows], rs[kLnBwdRows], s[2 * kLnBwdRows];
 #pragma unroll
-    for (int r = 0; r < kLnRows; ++r) {
-      float xv[8], dv[8], s1 = 0.f, s2 = 0.f;
-      unpack(xp[r], xv);
-      unpack(dp[r], dv);
+    for (int r = 0; r < kLnBwdRows; ++r) {
+      xp[r] = xn[r];
+      dp[r] = dn[r];
+      rp[r] = rn[r];
+      mu[r] = mun[r];
+      rs[r] = rsn[r];
+    }
+    load(row0 + step);
+    {
+      float xv[kLnBwdRows][8], dv[kLnBwdRows][8], s1[kLnBwdRows] = {}, s2[kLnBwdRows] = {};
+#pragma unroll
+      for (int r = 0; r < kLnBwdRows; ++r) {
+        unpack(xp[r], xv[r]);
+        unpack(dp[r], dv[r]);
+      }
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const float xh = (xv[k] - mu[r]) * rs[r], gy = dv[k] * g[k];
-        s1 = fmaf(gy, xh, s1);
-        s2 += gy;
-        dg[k] = fmaf(dv[k], xh, dg[k]);
-        db[k] += dv[k];
-      }
-      s[2 * r] = active ? s1 : 0.f;
-      s[2 * r + 1] = active ? s2 : 0.f;
-    }
-    cta_sum_many<2 * kLnRows>(s, red[buffer], warp, lane, warps);
+        float tg = 0.f, tb = 0.f;  // the rows meet before the long sums: half as many additions at their magnitude
 #pragma unroll
-    for (int r = 0; r < kLnRows; ++r) {
+        for (int r = 0; r < kLnBwdRows; ++r) {
+          const float xh = (xv[r][k] - mu[r]) * rs[r], gy = dv[r][k] * g[k];
+          s1[r] = fmaf(gy, xh, s1[r]);
+          s2[r] += gy;
+          tg = fmaf(dv[r][k], xh, tg);
+          tb += dv[r][k];
+        }
+        dg[k] += tg;
+        db[k] += tb;
+      }
+#pragma unroll
+      for (int r = 0; r < kLnBwdRows; ++r) {
+        s[2 * r] = active ? s1[r] : 0.f;
+        s[2 * r + 1] = active ? s2[r] : 0.f;
+      }
+    }
+    cta_sum_many<2 * kLnBwdRows>(s, red[buffer], warp, lane, warps);
+#pragma unroll
+    for (int r = 0; r < kLnBwdRows; ++r) {
       if (row0 + r >= rows || !active) break;
       const float c1 = s[2 * r] * inv_d, c2 = s[2 * r + 1] * inv_d;
       float xv[8], dv[8], o[8];
@@ -685,65 +717,67 @@ __global__ void __launch_bounds__(256, 2) ln_bwd_kernel(const __nv_bfloat16 *__r
   }
 }
 
-// Sums the CTAs' partial rows: 32 columns per block, a warp's lanes are eight groups of four columns times four rows. 128 threads
-// and 512 bytes of shared memory find room on an SM that a GEMM block holds; with more of either a launch waited for GEMM
-// blocks to retire (23 us a launch inside a training step, 15 with this).
+// Sums the CTAs' partial rows. These are up to 4.6 MB at every width (512 threads an SM with sixteen sums each), so a block takes
+// few columns and many rows at once: QUADS groups of four columns, 128 / QUADS rows. 32768 rows of 768: 10.5 -> 4.6 us, where 32
+// columns a block left 48 blocks to do it. Four columns (half of a 32-byte sector) are the better choice while eight would leave
+// fewer blocks than SMs: 32768 rows of 256 in 7.2 us with eight, 5.2 with four. 128 threads and 128 bytes of shared memory find room
+// on an SM that a GEMM block holds; with more of either a launch waited for GEMM blocks to retire.
+template <int QUADS>
 __global__ void __launch_bounds__(128) ln_bwd_reduce_kernel(const float *__restrict__ scratch, int parts, int d,
                                                             float *__restrict__ dgamma, float *__restrict__ dbeta, int accumulate) {
-  __shared__ float4 red[4][8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cq = lane & 7;
-  const int col = blockIdx.x * 32 + cq * 4;
+  __shared__ float4 red[4][QUADS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cq = lane % QUADS;
   const int which = blockIdx.y;  // 0 = dgamma, 1 = dbeta
+  const float *src = scratch + static_cast<int64_t>(which) * d + blockIdx.x * (4 * QUADS) + cq * 4;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (col < d) {
-    const float *src = scratch + static_cast<int64_t>(which) * d + col;
 #pragma unroll 8
-    for (int p = threadIdx.x >> 3; p < parts; p += 16) {
-      const float4 v = *reinterpret_cast<const float4 *>(src + static_cast<int64_t>(p) * 2 * d);
-      acc.x += v.x;
-      acc.y += v.y;
-      acc.z += v.z;
-      acc.w += v.w;
-    }
+  for (int p = threadIdx.x / QUADS; p < parts; p += 128 / QUADS) {
+    const float4 v = *reinterpret_cast<const float4 *>(src + static_cast<int64_t>(p) * 2 * d);
+    acc.x += v.x;
+    acc.y += v.y;
+    acc.z += v.z;
+    acc.w += v.w;
   }
 #pragma unroll
-  for (int o = 8; o <= 16; o <<= 1) {
+  for (int o = QUADS; o <= 16; o <<= 1) {
     acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
     acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
     acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
     acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
   }
-  if (lane < 8) red[warp][cq] = acc;
+  if (lane < QUADS) red[warp][cq] = acc;
   __syncthreads();
-  const int c = blockIdx.x * 32 + threadIdx.x;
-  if (threadIdx.x < 32 && c < d) {
-    float t = 0.f;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) t += reinterpret_cast<const float *>(red[w])[threadIdx.x];
+  if (threadIdx.x < 4 * QUADS) {
+    const int c = blockIdx.x * (4 * QUADS) + threadIdx.x;
+    const auto part = [&](int w) { return reinterpret_cast<const float *>(red[w])[threadIdx.x]; };
+    const float t = (part(0) + part(1)) + (part(2) + part(3));
     float *out = which == 0 ? dgamma : dbeta;
     out[c] = accumulate ? out[c] + t : t;
   }
 }
 
 int ln_threads(int d) { return (d / 8 + 31) / 32 * 32; }
-// CTAs: what the SMs hold at `per_sm_threads` threads each (64 registers a thread forward, 128 backward), but no more than
-// there are groups of rows or `most`.
-int64_t ln_grid(int64_t rows, int d, int per_sm_threads, int64_t most) {
-  const int fit = per_sm_threads / ln_threads(d);
-  const int64_t wave = static_cast<int64_t>(kSmCount) * (fit > 6 ? 6 : fit);
-  const int64_t groups = (rows + kLnRows - 1) / kLnRows, cap = wave < most ? wave : most;
+// CTAs of the column kernels: what the SMs hold at `per_sm_threads` threads each (64 registers a thread forward, 128 backward),
+// but no more than there are groups of rows or `most`.
+int64_t ln_grid(int64_t rows, int d, int group, int per_sm_threads, int64_t most) {
+  const int64_t wave = static_cast<int64_t>(kSmCount) * (per_sm_threads / ln_threads(d));
+  const int64_t groups = (rows + group - 1) / group, cap = wave < most ? wave : most;
   return groups < cap ? groups : cap;
 }
+constexpr int kLnBwdThreads = 512, kLnFwdThreads = 1024;  // per SM
 int launch_ln_bwd(cudaStream_t s, const void *dy, const void *x, const void *gamma, int pdt, const float *mean, const float *rstd,
                   const void *dres, void *dx, float *dgamma, float *dbeta, int accumulate, float *scratch, int64_t rows, int d,
                   int64_t scratch_rows) {
-  const int parts = static_cast<int>(ln_grid(rows, d, 512, scratch_rows));
+  const int parts = static_cast<int>(ln_grid(rows, d, kLnBwdRows, kLnBwdThreads, scratch_rows));
   ln_bwd_kernel<<<parts, ln_threads(d), 0, s>>>(static_cast<const __nv_bfloat16 *>(dy), static_cast<const __nv_bfloat16 *>(x), gamma,
                                                 pdt, mean, rstd, static_cast<const __nv_bfloat16 *>(dres),
                                                 static_cast<__nv_bfloat16 *>(dx), scratch, rows, d);
   const int code = finish_launch();
   if (code != 0) return code;
-  ln_bwd_reduce_kernel<<<dim3(static_cast<unsigned>((d + 31) / 32), 2), 128, 0, s>>>(scratch, parts, d, dgamma, dbeta, accumulate);
+  if (d / 8 * 2 < kSmCount)
+    ln_bwd_reduce_kernel<1><<<dim3(static_cast<unsigned>(d / 4), 2), 128, 0, s>>>(scratch, parts, d, dgamma, dbeta, accumulate);
+  else
+    ln_bwd_reduce_kernel<2><<<dim3(static_cast<unsigned>(d / 8), 2), 128, 0, s>>>(scratch, parts, d, dgamma, dbeta, accumulate);
   return finish_launch();
 }
 
@@ -771,12 +805,14 @@ int layernorm_forward(stream_t stream, const void *x, const void *gamma, const v
   if (chunks <= 3) return launch_ln_fwd_rows<3>(s, x, gamma, beta, param_dtype, y, mean, rstd, rows, di, eps);
   if (chunks > 16) return launch_ln_fwd_rows<32>(s, x, gamma, beta, param_dtype, y, mean, rstd, rows, di, eps);
   if (chunks > 8) return launch_ln_fwd_rows<16>(s, x, gamma, beta, param_dtype, y, mean, rstd, rows, di, eps);
-  ln_fwd_kernel<<<static_cast<int>(ln_grid(rows, di, 1024, rows)), ln_threads(di), 0, s>>>(
+  ln_fwd_kernel<<<static_cast<int>(ln_grid(rows, di, kLnRows, kLnFwdThreads, rows)), ln_threads(di), 0, s>>>(
       static_cast<const __nv_bfloat16 *>(x), gamma, beta, param_dtype, static_cast<__nv_bfloat16 *>(y), mean, rstd, rows, di, eps);
   return finish_launch();
 }
 
-int64_t layernorm_backward_scratch_rows() { return kLnBwdCtas; }
+int64_t layernorm_backward_scratch_rows(int64_t d) {
+  return static_cast<int64_t>(kSmCount) * (kLnBwdThreads / ln_threads(static_cast<int>(d)));
+}
 
 int layernorm_backward(stream_t stream, const void *dy, const void *x, const void *gamma, int param_dtype,
                        const float *mean, const float *rstd, const void *grad_residual, void *dx, float *dgamma,
@@ -785,7 +821,7 @@ int layernorm_backward(stream_t stream, const void *dy, const void *x, const voi
   if (d % 8 != 0 || d > 2048) return static_cast<int>(cudaErrorInvalidValue);  // wider rows use the library path
   if (rows == 0) return 0;
   return launch_ln_bwd(s, dy, x, gamma, param_dtype, mean, rstd, grad_residual, dx, dgamma, dbeta, accumulate, scratch, rows,
-                       static_cast<int>(d), kLnBwdCtas);
+                       static_cast<int>(d), layernorm_backward_scratch_rows(d));
 }
 
 // --------------------------------------------------------------------------- embedding ----

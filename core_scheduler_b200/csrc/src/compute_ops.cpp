@@ -698,7 +698,7 @@ Tensor layer_norm_backward_task(const Scheduler &scheduler, const std::shared_pt
              }
              at::Tensor dx = at::empty_like(x);
              at::Tensor scratch =
-                 at::empty({2 * kernels::layernorm_backward_scratch_rows() * d}, x.options().dtype(at::kFloat));
+                 at::empty({2 * kernels::layernorm_backward_scratch_rows(d) * d}, x.options().dtype(at::kFloat));
              task.intermediate().push_back(scratch);
              at::Tensor r2;
              if (res) r2 = cast_if(res->impl()->tensor, at::kBFloat16).contiguous();
