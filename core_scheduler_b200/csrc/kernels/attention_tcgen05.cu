@@ -444,28 +444,30 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS_PER_SM) attention_fwd_kernel
     }
     // the last block's P V completes the accumulator
     const bool done = ok && mbar_wait_warp(bar(O_DONE), (num_kv - 1) & 1, abort_flag);
-    if (done && !*abort_flag && q_idx < p.T &&
-        CS_IN_BOUNDS(kKidAttention, (static_cast<long long>(row_base + q_idx) * p.H + h) * HD + HD - 1,
-                     static_cast<long long>(p.B) * p.T * p.H * HD)) {
+    if (__all_sync(0xffffffffu, done && !*abort_flag)) {
       fence_after();
-      const float inv = 1.f / l_run;
-      __nv_bfloat16 *dst = p.out + (static_cast<long long>(row_base + q_idx) * p.H + h) * HD;
       uint32_t o[2][32];
       tmem_ld32(o_tmem + lane_addr, o[0]);
       tmem_ld32(o_tmem + 32 + lane_addr, o[1]);
       tmem_wait_ld();
+      const bool row_in_range = CS_IN_BOUNDS(kKidAttention, (static_cast<long long>(row_base + q_idx) * p.H + h) * HD + HD - 1,
+                                             static_cast<long long>(p.B) * p.T * p.H * HD);
+      const float inv = 1.f / l_run;
+      __nv_bfloat16 *dst = p.out + (static_cast<long long>(row_base + q_idx) * p.H + h) * HD;
+      if (row_in_range) {
 #pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        const uint32_t(&w8)[32] = o[g >> 2];
-        const int at = (g & 3) * 8;
-        uint4 w;
-        w.x = pack2(__uint_as_float(w8[at + 0]) * inv, __uint_as_float(w8[at + 1]) * inv);
-        w.y = pack2(__uint_as_float(w8[at + 2]) * inv, __uint_as_float(w8[at + 3]) * inv);
-        w.z = pack2(__uint_as_float(w8[at + 4]) * inv, __uint_as_float(w8[at + 5]) * inv);
-        w.w = pack2(__uint_as_float(w8[at + 6]) * inv, __uint_as_float(w8[at + 7]) * inv);
-        *reinterpret_cast<uint4 *>(dst + g * 8) = w;
+        for (int g = 0; g < 8; ++g) {
+          const uint32_t(&w8)[32] = o[g >> 2];
+          const int at = (g & 3) * 8;
+          uint4 w;
+          w.x = pack2(__uint_as_float(w8[at + 0]) * inv, __uint_as_float(w8[at + 1]) * inv);
+          w.y = pack2(__uint_as_float(w8[at + 2]) * inv, __uint_as_float(w8[at + 3]) * inv);
+          w.z = pack2(__uint_as_float(w8[at + 4]) * inv, __uint_as_float(w8[at + 5]) * inv);
+          w.w = pack2(__uint_as_float(w8[at + 6]) * inv, __uint_as_float(w8[at + 7]) * inv);
+          *reinterpret_cast<uint4 *>(dst + g * 8) = w;
+        }
+        p.lse[(static_cast<long long>(b) * p.H + h) * p.T + q_idx] = m_run * p.scale + __logf(l_run);
       }
-      p.lse[(static_cast<long long>(b) * p.H + h) * p.T + q_idx] = m_run * p.scale + __logf(l_run);
     }
   }
 

@@ -390,7 +390,7 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
       if constexpr (epi_uses_aux<EPI>) {
         if (sub == 0) {
           box = st.base + (ch >> 1) * EPI_BUF_BYTES;
-          if (!__all_sync(0xffffffffu, mbar_wait(aux_bar + 8u * (ch >> 1), aux_parity, abort_flag))) {
+          if (!mbar_wait_warp(aux_bar + 8u * (ch >> 1), aux_parity, abort_flag)) {
             tcgen05_wait_ld();  // no load may be outstanding when the kernel unwinds
             return false;
           }
@@ -816,7 +816,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
       for (int tile = pair; tile < total_tiles; tile += num_pairs) {
         const TileCoord c = tile_coord2<TN>(p, tile);
         const int m0_cta = c.m0 + static_cast<int>(cta) * 128;
-        if (!mbar_wait(tmem_full_bar(acc), acc_phase, abort_flag)) break;
+        if (!mbar_wait_warp(tmem_full_bar(acc), acc_phase, abort_flag)) break;
         tcgen05_fence_after();
         auto release = [&] {
           tcgen05_fence_before();
