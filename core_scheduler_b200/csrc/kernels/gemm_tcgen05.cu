@@ -352,7 +352,7 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
   const uint32_t taddr = tmem_acc + col_base + (static_cast<uint32_t>(q * 32) << 16);
   uint32_t acc[2][32];
   tcgen05_ld_32x32b_x32(taddr, acc[0]);
-  float run_max = -INFINITY, run_sum = 0.f;  // base-2 softmax partials
+  float run_max = -INFINITY, run_sum = 0.f;  // softmax partials
   uint32_t box = 0;
 #pragma unroll
   for (int ch = 0; ch < CHUNKS; ++ch) {
@@ -436,49 +436,52 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
                          activated[4 * g + 3]);
         }
         if constexpr (EPI == kEpiCrossEntropy) {
-          // running (max, sum-exp) over the valid columns, on the logits as stored (bf16)
+          // Running (max, sum-exp) over the valid columns, on the logits as stored (bf16). Exponents are differences to the
+          // maximum times log2(e), not a product minus a product: the maximum stays the bf16 value it is, and neither
+          // rounding nor overflow of the products gets into the sum.
           constexpr float kLog2e = 1.4426950408889634f;
           const long long left = p.n_valid - gcol;  // valid columns of this chunk
+          auto raise = [&](float cmax) {
+            if (cmax > run_max) {
+              run_sum *= ex2_approx((run_max - cmax) * kLog2e);  // first chunk: 0 * exp2(-inf) = 0
+              run_max = cmax;
+            }
+          };
           if (left >= 32) {
             __nv_bfloat162 mx = *reinterpret_cast<__nv_bfloat162 *>(&packed[0]);
 #pragma unroll
             for (int i = 1; i < 16; ++i) mx = __hmax2(mx, *reinterpret_cast<__nv_bfloat162 *>(&packed[i]));
-            const float cmax = fmaxf(__low2float(mx), __high2float(mx)) * kLog2e;
-            if (cmax > run_max) {
-              run_sum *= ex2_approx(run_max - cmax);  // first chunk: 0 * exp2(-inf) = 0
-              run_max = cmax;
-            }
+            const float cmax = fmaxf(__low2float(mx), __high2float(mx));
+            raise(cmax);
             if (run_max > -INFINITY) {
-            const F2 scale = f2(kLog2e, kLog2e), shift = f2(-run_max, -run_max);
-            F2 s0 = f2(0.f, 0.f), s1 = f2(0.f, 0.f);
+              const F2 scale = f2(kLog2e, kLog2e), shift = f2(-run_max, -run_max);
+              F2 s0 = f2(0.f, 0.f), s1 = f2(0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-              float a, b, c, d;
-              f2_split(f2_fma(f2_unpack_bf16(packed[i]), scale, shift), a, b);
-              f2_split(f2_fma(f2_unpack_bf16(packed[i + 1]), scale, shift), c, d);
-              s0 = f2_add(s0, f2(ex2_approx(a), ex2_approx(b)));
-              s1 = f2_add(s1, f2(ex2_approx(c), ex2_approx(d)));
-            }
-            float a, b;
-            f2_split(f2_add(s0, s1), a, b);
-            run_sum += a + b;
+              for (int i = 0; i < 16; i += 2) {
+                float a, b, c, d;
+                f2_split(f2_mul(f2_add(f2_unpack_bf16(packed[i]), shift), scale), a, b);
+                f2_split(f2_mul(f2_add(f2_unpack_bf16(packed[i + 1]), shift), scale), c, d);
+                s0 = f2_add(s0, f2(ex2_approx(a), ex2_approx(b)));
+                s1 = f2_add(s1, f2(ex2_approx(c), ex2_approx(d)));
+              }
+              float a, b;
+              f2_split(f2_add(s0, s1), a, b);
+              run_sum += a + b;
             }
           } else if (left > 0) {
             float cmax = -INFINITY;
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-              const float x = __uint_as_float(i & 1 ? packed[i >> 1] & 0xffff0000u : packed[i >> 1] << 16) * kLog2e;
+              const float x = __uint_as_float(i & 1 ? packed[i >> 1] & 0xffff0000u : packed[i >> 1] << 16);
               if (i < left) cmax = fmaxf(cmax, x);
             }
-            if (cmax > run_max) {
-              run_sum *= ex2_approx(run_max - cmax);
-              run_max = cmax;
-            }
-            if (run_max > -INFINITY)
+            raise(cmax);
+            if (run_max > -INFINITY) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const float x = __uint_as_float(i & 1 ? packed[i >> 1] & 0xffff0000u : packed[i >> 1] << 16);
-              if (i < left) run_sum += ex2_approx(fmaf(x, kLog2e, -run_max));
+              for (int i = 0; i < 32; ++i) {
+                const float x = __uint_as_float(i & 1 ? packed[i >> 1] & 0xffff0000u : packed[i >> 1] << 16);
+                if (i < left) run_sum += ex2_approx((x - run_max) * kLog2e);
+              }
             }
           }
         }
@@ -495,7 +498,7 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
     const long long row = row0 + lane;
     if (row < p.m) {
       float *stp = p.stats + (row * (2LL * p.n_tiles) + 2LL * n_tile + half) * 2;
-      stp[0] = run_max * 0.69314718055994530942f;  // natural logarithm, as the merging kernels expect
+      stp[0] = run_max;
       stp[1] = run_sum;
     }
   }

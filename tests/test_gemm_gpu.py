@@ -166,3 +166,24 @@ def test_gelu_epilogue_limits():
     assert C.gemm_bf16(a, b, d, TN, GELU_DUAL, d2=d2, bias=None) == 0
     big = b[1, 0].item()
     assert d2[7, 1].item() == big and d2[7, 2].item() == 0 and d2[7, 3].item() == 0 and d2[7, 4].item() == 20
+
+
+@pytest.mark.parametrize("spread", [1.0, 100.0, 3e37])
+@pytest.mark.parametrize("M,N,n_valid", [(130, 512, 512), (64, 640, 600), (256, 136, 130)])
+def test_softmax_partials_hold_the_exact_maximum(M, N, n_valid, spread):
+    """(max, sum-exp) of every 128-column half tile: the maximum is the stored logit itself, the sum that of exp(x - max), at
+    magnitudes up to where a product with log2(e) overflows. ex2.approx is within 2 ulp, 2^-22; at most 128 fp32 additions."""
+    torch.manual_seed(M + N)
+    a, b = torch.zeros(M, 64, device="cuda", dtype=BF), (torch.randn(N, 64, device="cuda") * spread).to(BF)
+    a[torch.arange(M), torch.arange(M) % 64] = 1  # each row of logits is a column of b
+    d = torch.empty(M, N, device="cuda", dtype=BF)
+    tiles = 2 * ((N + 255) // 256)
+    stats = torch.full((M, tiles, 2), 7.0, device="cuda")
+    assert C.gemm_bf16(a, b, d, TN, 6, stats=stats, n_valid=n_valid) == 0
+    x = d.double()
+    x[:, n_valid:] = float("-inf")
+    x = torch.nn.functional.pad(x, (0, tiles * 128 - N), value=float("-inf")).view(M, tiles, 128)
+    mx = x.amax(-1)
+    assert torch.equal(stats[..., 0].double(), mx)
+    want = torch.where(mx > float("-inf"), (x - mx[..., None]).exp().sum(-1), torch.zeros_like(mx))
+    assert ((stats[..., 1].double() - want).abs() <= (128 * 2.0 ** -24 + 2.0 ** -20) * want).all()
