@@ -1032,12 +1032,12 @@ __device__ __forceinline__ void merge_softmax_partials(const float *st, int n_ti
   for (int i = 0; i < kHeld; ++i) mx = fmaxf(mx, held[i].x);
   for (int t = lane + 32 * kHeld; t < n_tiles; t += 32) mx = fmaxf(mx, pairs[t].x);
   mx = warp_max(mx);
+  // a tile without a maximum has the sum 0, or NaN where its logits are
+  const auto rescaled = [mx](float2 pair) { return pair.x > -INFINITY ? pair.y * __expf(pair.x - mx) : pair.y; };
   float sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < kHeld; ++i)
-    if (held[i].x > -INFINITY) sum += held[i].y * __expf(held[i].x - mx);
-  for (int t = lane + 32 * kHeld; t < n_tiles; t += 32)
-    if (pairs[t].x > -INFINITY) sum += pairs[t].y * __expf(pairs[t].x - mx);
+  for (int i = 0; i < kHeld; ++i) sum += rescaled(held[i]);
+  for (int t = lane + 32 * kHeld; t < n_tiles; t += 32) sum += rescaled(pairs[t]);
   mx_out = mx;
   sum_out = warp_sum(sum);
 }
@@ -1171,7 +1171,7 @@ __global__ void __launch_bounds__(256) ce_slice_stats_kernel(const float *__rest
   float mx, sum;
   merge_softmax_partials(stats + row * n_tiles * 2, static_cast<int>(n_tiles), lane, mx, sum);
   if (lane == 0) {
-    out[row * 2] = (n_valid_local > 0 && mx > -INFINITY) ? mx + __logf(sum) : -INFINITY;
+    out[row * 2] = (n_valid_local > 0 && (mx > -INFINITY || sum != 0.f)) ? mx + __logf(sum) : -INFINITY;
     const int64_t local = target[row] - col_offset;
     out[row * 2 + 1] = (local >= 0 && local < n_valid_local) ? __bfloat162float(logits[row * ld + local]) : 0.f;
   }

@@ -467,13 +467,18 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
               float a, b;
               f2_split(f2_add(s0, s1), a, b);
               run_sum += a + b;
+            } else if (cmax != cmax) {
+              run_sum = cmax;  // nothing but NaN so far: no maximum, but not an empty chunk either
             }
           } else if (left > 0) {
-            float cmax = -INFINITY;
+            float cmax = -INFINITY, nan = 0.f;
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               const float x = __uint_as_float(i & 1 ? packed[i >> 1] & 0xffff0000u : packed[i >> 1] << 16);
-              if (i < left) cmax = fmaxf(cmax, x);
+              if (i < left) {
+                cmax = fmaxf(cmax, x);
+                if (x != x) nan = x;
+              }
             }
             raise(cmax);
             if (run_max > -INFINITY) {
@@ -482,6 +487,8 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
                 const float x = __uint_as_float(i & 1 ? packed[i >> 1] & 0xffff0000u : packed[i >> 1] << 16);
                 if (i < left) run_sum += ex2_approx((x - run_max) * kLog2e);
               }
+            } else if (nan != nan) {
+              run_sum = nan;
             }
           }
         }

@@ -405,3 +405,21 @@ def test_layernorm_where_its_dispatch_changes(gpu_scheduler, rows, d):
     """Around 768 columns (a warp or a CTA per row forward), 592 (columns per block of the gradient sum) and a multiple of 256,
     with odd row counts below and above one wave of CTAs: the bounds of the test above."""
     test_layernorm_column_kernels(gpu_scheduler, rows, d)
+
+
+@pytest.mark.parametrize("first,last", [(0, 32), (0, 128), (64, 96), (0, 512), (480, 500)])
+def test_nan_logits_of_whole_chunks_reach_the_loss(gpu_scheduler, first, last):
+    """NaN in all logits of one 32-column chunk, of a half tile, of every column, or of the last columns before the end of the
+    vocabulary (the epilogue looks at 32 columns at a time): the row's loss is NaN, as log_softmax has it."""
+    s = gpu_scheduler
+    torch.manual_seed(0)
+    lin = C.linear_init(s, 64, 512, bias=False)
+    s.synchronize()
+    lin.weight.raw()[first:last] = float("nan")
+    ce = C.linear_cross_entropy_init(s, lin, valid_classes=500)
+    x = torch.randn(40, 64, device="cuda").to(BF)
+    target = torch.full((40,), 300, device="cuda")
+    with cs.autocast(s, BF):
+        loss = C.linear_cross_entropy_forward(s, ce, T(x), T(target))
+    s.synchronize()
+    assert torch.isnan(loss.raw()).all()
