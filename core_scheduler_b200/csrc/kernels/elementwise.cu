@@ -1125,7 +1125,7 @@ __global__ void __launch_bounds__(256) ce_backward_kernel(__nv_bfloat16 *__restr
         } else {
           unpack(v[u], f);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(f[k]) : "f"(fmaf(f[k], log2e, -l2)));
+          for (int k = 0; k < 8; ++k) f[k] = exp2f(fmaf(f[k], log2e, -l2));  // subnormal probabilities are gradients too
           if (col + 8 > valid) {
 #pragma unroll
             for (int k = 0; k < 8; ++k)

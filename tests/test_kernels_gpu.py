@@ -423,3 +423,25 @@ def test_nan_logits_of_whole_chunks_reach_the_loss(gpu_scheduler, first, last):
         loss = C.linear_cross_entropy_forward(s, ce, T(x), T(target))
     s.synchronize()
     assert torch.isnan(loss.raw()).all()
+
+
+def test_classifier_gradient_keeps_subnormal_probabilities(gpu_scheduler):
+    """One row with logits 0 .. -100: probabilities down to 2^-133, bf16's smallest number, come back as gradients. bf16 keeps
+    fewer bits there: half of 2^-133 beside 2^-8 of the value."""
+    s = gpu_scheduler
+    lin = C.linear_init(s, 64, 64, bias=False)
+    s.synchronize()
+    w = lin.weight.raw()
+    w.zero_()
+    w[:, 0] = torch.linspace(0, -100, 64, device="cuda")
+    ce = C.linear_cross_entropy_init(s, lin)
+    x = torch.zeros(1, 64, device="cuda", dtype=BF)
+    x[0, 0] = 1
+    with cs.autocast(s, BF):
+        C.linear_cross_entropy_forward(s, ce, T(x), T(torch.zeros(1, dtype=torch.int64, device="cuda")))
+    C.linear_cross_entropy_backward(s, ce)
+    s.synchronize()
+    p = torch.softmax(w[:, 0].to(BF).double(), 0)[1:]
+    got = lin.grad_weight.raw()[1:, 0].double()
+    assert ((got - p).abs() <= 2.0 ** -8 * p + 2.0 ** -133 * 0.51).all()
+    assert (got[p > 2.0 ** -132] > 0).all()
