@@ -445,3 +445,30 @@ def test_classifier_gradient_keeps_subnormal_probabilities(gpu_scheduler):
     got = lin.grad_weight.raw()[1:, 0].double()
     assert ((got - p).abs() <= 2.0 ** -8 * p + 2.0 ** -133 * 0.51).all()
     assert (got[p > 2.0 ** -132] > 0).all()
+
+
+@pytest.mark.parametrize("rows,vocab,padded", [(3, 7, 8), (70, 300, 304), (2500, 512, 512), (33, 1000, 1000), (9, 7160, 7160), (9, 8190, 8192), (9, 8200, 8200)])
+def test_classifier_loss_over_vocabulary_sizes(gpu_scheduler, rows, vocab, padded):
+    """Rows of less than one chunk a thread, the last width with fewer than 256 threads, 64 and 66 softmax partials a row, more rows
+    than CTAs. The reference starts from the bf16 logits, so that the loss is left with fp32 sums (and logits that round the
+    other way: 2^-9 of one in a few); gradients are bf16, 5e-3 in the norm."""
+    s = gpu_scheduler
+    torch.manual_seed(rows + vocab)
+    lin = C.linear_init(s, 64, padded, bias=False)
+    ce = C.linear_cross_entropy_init(s, lin, valid_classes=vocab)
+    x, target = torch.randn(rows, 64, device="cuda").to(BF), torch.randint(0, vocab, (rows,), device="cuda")
+    target[0] = vocab - 1
+    s.synchronize()
+    with cs.autocast(s, BF):
+        loss = C.linear_cross_entropy_forward(s, ce, T(x), T(target))
+    dx = C.linear_cross_entropy_backward(s, ce)
+    s.synchronize()
+    w = lin.weight.raw().to(BF).double()
+    logits = (x.double() @ w[:vocab].t()).to(BF).double().requires_grad_(True)
+    ref = F.cross_entropy(logits, target)
+    ref.backward()
+    assert abs(loss.raw().double().item() - ref.item()) < 1e-4 * max(1.0, ref.item())
+    dw = torch.zeros_like(w)
+    dw[:vocab] = logits.grad.t() @ x.double()
+    assert ((dx.raw().double() - logits.grad @ w[:vocab]).norm() / (logits.grad @ w[:vocab]).norm()).item() < 5e-3
+    assert ((lin.grad_weight.raw().double() - dw).norm() / dw.norm()).item() < 5e-3
