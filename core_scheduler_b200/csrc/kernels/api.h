@@ -99,6 +99,7 @@ struct GemmArgs {
   const void *aux;   // residual / pre-activation, same shape & leading dim as d
   const void *bias;  // bf16 [N] or nullptr
   float *stats;      // kEpiCrossEntropy: [M, gemm_ce_stat_tiles(N), 2] (max, sum-exp) partials
+  int64_t stats_len; // floats in `stats` (looked at by the diagnostic build)
   int64_t m, n, k;
   int64_t lda, ldb, ldd;
   int layout;

@@ -47,12 +47,10 @@ constexpr int THREADS = 64 + EPI_WARPS * 32;
 constexpr long long kWaitBudgetCycles = 4000000000LL;  // ~2 s at 2 GHz
 
 struct KParams {
-  void *d;
-  void *d2;
-  const void *aux;
   const void *bias;
   float *stats;
-  long long m, n, k, ldd, n_valid;
+  long long stats_len;  // floats in `stats`
+  long long m, n, n_valid;
   int layout, epilogue;
   int m_tiles, n_tiles, splits, kb_total, kb_per_split;
   int group_m;         // pair kernel: row tiles that are walked together before the next column tile
@@ -503,8 +501,9 @@ __device__ __forceinline__ bool epilogue_pair_tile(const KParams &p, const CUten
   }
   if constexpr (EPI == kEpiCrossEntropy) {
     const long long row = row0 + lane;
-    if (row < p.m) {
-      float *stp = p.stats + (row * (2LL * p.n_tiles) + 2LL * n_tile + half) * 2;
+    const long long at = (row * (2LL * p.n_tiles) + 2LL * n_tile + half) * 2;
+    if (row < p.m && CS_IN_BOUNDS(kKidGemmEpilogue, at + 1, p.stats_len)) {
+      float *stp = p.stats + at;
       stp[0] = run_max;
       stp[1] = run_sum;
     }
@@ -614,9 +613,9 @@ __device__ __forceinline__ TileCoord tile_coord2(const KParams &p, int tile) {
   return c;
 }
 
-// 128 registers per thread (no spills): the SM's four register files are filled by warps, and a partition that
-// holds three of this block's ten warps then still has room for two warps of a light kernel (collectives, AdamW),
-// so those really run beside a resident GEMM block instead of waiting for it to retire.
+// 128 registers per thread (the two wide forms with both GELU outputs spill 16 and 24 bytes at it): the SM's four register
+// files are filled by warps, and a partition that holds three of this block's ten warps then still has room for two warps of a
+// light kernel (collectives, AdamW), so those really run beside a resident GEMM block instead of waiting for it to retire.
 // map_aux: auxiliary operand in output boxes (epilogues that have one); map_d2: second output (kEpiGeluDual).
 template <int TN, int EPI>
 __global__ void __maxnreg__(128)
@@ -936,11 +935,12 @@ cudaError_t launch_pair_epi(int epi, cudaStream_t s, int grid, const CUtensorMap
     case kEpiResidualBf16: return launch_pair<TN, kEpiResidualBf16>(s, grid, a, b, d, d2, peers, p);
     case kEpiGeluDual: return launch_pair<TN, kEpiGeluDual>(s, grid, a, b, d, d2, peers, p);
     case kEpiDGelu: return launch_pair<TN, kEpiDGelu>(s, grid, a, b, d, d2, peers, p);
-    case kEpiStoreF32:
-    case kEpiAccumF32: return launch_pair<TN, kEpiStoreF32>(s, grid, a, b, d, d2, peers, p);
     default: break;
   }
-  if constexpr (TN == 256) return launch_pair<TN, kEpiCrossEntropy>(s, grid, a, b, d, d2, peers, p);
+  if constexpr (TN == 256) {  // choose_tile_n narrows bf16 outputs only, and not the classifier's
+    if (epi == kEpiStoreF32 || epi == kEpiAccumF32) return launch_pair<TN, kEpiStoreF32>(s, grid, a, b, d, d2, peers, p);
+    if (epi == kEpiCrossEntropy) return launch_pair<TN, kEpiCrossEntropy>(s, grid, a, b, d, d2, peers, p);
+  }
   return cudaErrorInvalidValue;
 }
 
@@ -1057,15 +1057,11 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
   if (a.epilogue == kEpiGeluDual && !get_tensor_map(a.d2, a.n, a.m, a.ldd, 64, 32, &map_d2)) return -1;
 
   KParams p{};
-  p.d = a.d;
-  p.d2 = a.d2;
-  p.aux = a.aux;
   p.bias = a.bias;
   p.stats = a.stats;
+  p.stats_len = a.stats_len;
   p.m = a.m;
   p.n = a.n;
-  p.k = a.k;
-  p.ldd = a.ldd;
   p.n_valid = a.n_valid > 0 ? a.n_valid : a.n;
   p.layout = a.layout;
   p.epilogue = a.epilogue;

@@ -101,7 +101,7 @@ PYBIND11_MODULE(_C, m) {
           if (!aux.is_none()) { aux_t = py::cast<at::Tensor>(aux); g.aux = aux_t.data_ptr(); }
           if (!bias.is_none()) { bias_t = py::cast<at::Tensor>(bias); g.bias = bias_t.data_ptr(); }
           if (!d2.is_none()) { d2_t = py::cast<at::Tensor>(d2); g.d2 = d2_t.data_ptr(); }
-          if (!stats.is_none()) { stats_t = py::cast<at::Tensor>(stats); g.stats = stats_t.data_ptr<float>(); }
+          if (!stats.is_none()) { stats_t = py::cast<at::Tensor>(stats); g.stats = stats_t.data_ptr<float>(); g.stats_len = stats_t.numel(); }
           g.layout = layout;
           g.epilogue = epilogue;
           if (layout == cs::kernels::kTN) {

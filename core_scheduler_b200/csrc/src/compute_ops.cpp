@@ -1126,6 +1126,7 @@ Tensor LinearCrossEntropy::forward(const Scheduler &scheduler, const std::shared
              g.b = wc.data_ptr();
              g.d = lg.data_ptr();
              g.stats = stats.data_ptr<float>();
+             g.stats_len = stats.numel();
              g.m = rows;
              g.n = V;
              g.k = x2.size(1);

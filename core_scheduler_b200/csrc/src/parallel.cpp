@@ -873,6 +873,7 @@ Tensor TPGPT2Impl::forward_loss(const Scheduler &scheduler, const ReadOnlyTensor
              g.b = wc.data_ptr();
              g.d = lg.data_ptr();
              g.stats = partials.data_ptr<float>();
+             g.stats_len = partials.numel();
              g.m = M;
              g.n = classes;
              g.k = xf.size(1);

@@ -82,3 +82,37 @@ def test_checked_build_records_and_skips_out_of_range_indices():
     env = dict(os.environ, CS_BOUNDS_CHECK="1", CS_NO_AUTOBUILD="1", PYTHONPATH=ROOT)
     proc = subprocess.run([sys.executable, "-c", CHILD], env=env, capture_output=True, text=True, timeout=600)
     assert proc.returncode == 0 and "OK bounds" in proc.stdout, (proc.stdout + proc.stderr)[-3000:]
+
+
+STATS_CHILD = textwrap.dedent(
+    """
+    import torch
+    import core_scheduler_b200 as cs
+    C = cs._C
+    assert C.bounds_check_enabled(), "checked kernels not loaded"
+    BF = torch.bfloat16
+    a, b = torch.randn(200, 64, device="cuda").to(BF), torch.randn(512, 64, device="cuda").to(BF)
+    d = torch.empty(200, 512, device="cuda", dtype=BF)
+    whole = torch.full((200, 4, 2), 7.0, device="cuda")
+    assert C.gemm_bf16(a, b, d, 0, 6, stats=whole, n_valid=512) == 0
+    torch.cuda.synchronize()
+    assert C.bounds_report(True)[0] == 0 and not (whole == 7).any()
+    # the statistics buffer is declared shorter than the rows need; the memory behind it is there all the same
+    short = torch.full((200, 4, 2), 7.0, device="cuda")
+    assert C.gemm_bf16(a, b, d, 0, 6, stats=short[:150], n_valid=512) == 0
+    torch.cuda.synchronize()
+    code, kid, block, thread, index, limit = C.bounds_report(True)
+    assert (code, kid, limit) == (1, 19, 150 * 8) and limit <= index < 200 * 8, (code, kid, index, limit)
+    assert torch.equal(short[:150], whole[:150]) and (short[150:] == 7).all()
+    print("OK stats")
+    """
+)
+
+
+def test_checked_build_guards_the_classifier_statistics():
+    lib = os.path.join(ROOT, "core_scheduler_b200", "lib_checked", "libcs_b200.so")
+    if not os.path.exists(lib):
+        pytest.skip("diagnostic library not built (python -m core_scheduler_b200.build checked)")
+    env = dict(os.environ, CS_BOUNDS_CHECK="1", CS_NO_AUTOBUILD="1", PYTHONPATH=ROOT)
+    proc = subprocess.run([sys.executable, "-c", STATS_CHILD], env=env, capture_output=True, text=True, timeout=600)
+    assert proc.returncode == 0 and "OK stats" in proc.stdout, (proc.stdout + proc.stderr)[-3000:]

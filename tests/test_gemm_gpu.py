@@ -156,15 +156,16 @@ def test_narrow_tiles_with_every_epilogue(M, N, K, layout):
 
 
 def test_gelu_epilogue_limits():
-    """Infinite and very large pre-activations: GELU is x on the right and zero on the left, never NaN."""
+    """Infinite and very large pre-activations of either sign: GELU is x on the right and zero on the left, never NaN."""
     a = torch.zeros(256, 64, device="cuda", dtype=BF)
     a[:, 0] = 1
     b = torch.zeros(256, 64, device="cuda", dtype=BF)
-    b[:5, 0] = torch.tensor([float("inf"), 3e38, -3e38, -20.0, 20.0])
+    b[:6, 0] = torch.tensor([float("inf"), 3e38, -3e38, -20.0, 20.0, float("-inf")])
     d, d2 = torch.empty(256, 256, device="cuda", dtype=BF), torch.empty(256, 256, device="cuda", dtype=BF)
-    b[0, 1:] = 0
     assert C.gemm_bf16(a, b, d, TN, GELU_DUAL, d2=d2, bias=None) == 0
     big = b[1, 0].item()
+    assert torch.equal(d[7, :6], b[:6, 0]) and not d2.isnan().any()
+    assert d2[7, 0].item() == float("inf") and d2[7, 5].item() == 0
     assert d2[7, 1].item() == big and d2[7, 2].item() == 0 and d2[7, 3].item() == 0 and d2[7, 4].item() == 20
 
 
