@@ -944,17 +944,46 @@ cudaError_t launch_pair_epi(int epi, cudaStream_t s, int grid, const CUtensorMap
   return cudaErrorInvalidValue;
 }
 
+// Weight gradients have few output tiles and a long reduction: split K so that every SM has work; partial sums meet in the
+// fp32 output through vector atomics. The split count whose tile total fills whole waves of the pairs best, with at least 8
+// k-blocks per split; ties go to fewer splits (fewer reduce-adds).
+int64_t choose_splits(int64_t tiles, int64_t k_blocks, int pairs) {
+  int64_t best = 1;
+  double best_eff = 0.0;
+  for (int64_t sp = 1; sp <= k_blocks / 8 || sp == 1; ++sp) {
+    const int64_t total = tiles * sp, waves = (total + pairs - 1) / pairs;
+    const double eff = static_cast<double>(total) / (static_cast<double>(waves) * pairs);
+    if (eff > best_eff + 0.02) {
+      best_eff = eff;
+      best = sp;
+    }
+    if (total >= 4 * pairs || sp == 64) break;
+  }
+  return best;
+}
+
 // Width of the pair kernel's tile. A k-block of 64 costs a pair 2 TN cycles of tensor core or 256 + TN cycles of operand
 // traffic (64 bytes a cycle and SM, what the 8192^3 product sustains), whichever is more; a narrower tile pays only where
 // the wide ones leave pairs without work. Measured with 256 / 128 / 64 columns: 1536x768x3072 21.2 / 13.6 / 13.4 us,
 // 1536x2304x768 10.8 / 10.6 / 12.0, 3000x5120x1280 42.0 / 43.5 / 57.2, 16384x768x3072 60.5 / 65.9 / 92.6.
+//
+// An input gradient (kTM) runs beside the weight gradient of its layer, which is as large the other way round. Where that
+// leaves pairs free and 256-column tiles fit into them, narrower ones that do not only make the two take turns: forward and
+// backward of 1200 x 1024 x 3072 take 43 us with 40 narrow tiles beside 48, 37 with 20 wide ones (1500 x 768 x 2304: 38 and 32.5).
 int choose_tile_n(const GemmArgs &a, int pairs, bool fixed) {
   if (fixed) return 256;
   int best = 256;
   double best_cost = 0;
+  int64_t beside = INT64_MAX;  // tiles that narrowing may lead to
+  if (a.layout == kTM) {
+    const int64_t blocks = (a.k + BM2 - 1) / BM2 * ((a.n + BN - 1) / BN);
+    const int64_t free_pairs = pairs - blocks * choose_splits(blocks, (a.m + BK - 1) / BK, pairs);
+    if ((a.m + BM2 - 1) / BM2 * ((a.n + BN - 1) / BN) <= free_pairs) beside = free_pairs;
+  }
   for (int tn = 256; tn >= 64; tn /= 2) {
     if (tn == 64 && a.layout != kTN) break;  // an MN-major half tile of 32 columns is no whole swizzle atom
     const int64_t tiles = ((a.m + BM2 - 1) / BM2) * ((a.n + tn - 1) / tn);
+    if (tn < 256 && tiles > beside) break;
     const int64_t waves = (tiles + pairs - 1) / pairs;
     const double cost = static_cast<double>(waves) * (2 * tn > 256 + tn ? 2 * tn : 256 + tn);
     if (tn == 256 || cost < 0.95 * best_cost) {
@@ -1071,26 +1100,7 @@ int gemm_bf16(stream_t stream, const GemmArgs &a) {
   p.kb_total = static_cast<int>((a.k + BK - 1) / BK);
   p.splits = 1;
   if (f32_out) {
-    // Weight gradients have few output tiles and a long reduction: split K so that every SM
-    // has work; partial sums meet in the fp32 output through vector atomics.
-    const int mn = p.m_tiles * p.n_tiles;
-    const int workers = sm_count / 2;
-    // Pick the split count whose tile total fills whole waves of `workers` best, keeping at
-    // least 8 k-blocks per split; ties go to fewer splits (fewer reduce-adds).
-    const int max_splits = p.kb_total / 8 > 0 ? p.kb_total / 8 : 1;
-    int best = 1;
-    double best_eff = 0.0;
-    for (int sp = 1; sp <= max_splits && sp <= 64; ++sp) {
-      const int tiles = mn * sp;
-      const int waves = (tiles + workers - 1) / workers;
-      const double eff = static_cast<double>(tiles) / (static_cast<double>(waves) * workers);
-      if (eff > best_eff + 0.02) {
-        best_eff = eff;
-        best = sp;
-      }
-      if (tiles >= 4 * workers) break;
-    }
-    p.splits = best;
+    p.splits = static_cast<int>(choose_splits(static_cast<int64_t>(p.m_tiles) * p.n_tiles, p.kb_total, sm_count / 2));
   }
   p.kb_per_split = (p.kb_total + p.splits - 1) / p.splits;
   p.splits = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;

@@ -188,3 +188,18 @@ def test_softmax_partials_hold_the_exact_maximum(M, N, n_valid, spread):
     assert torch.equal(stats[..., 0].double(), mx)
     want = torch.where(mx > float("-inf"), (x - mx[..., None]).exp().sum(-1), torch.zeros_like(mx))
     assert ((stats[..., 1].double() - want).abs() <= (128 * 2.0 ** -24 + 2.0 ** -20) * want).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(844, 1024, 3072), (1200, 1024, 3072), (1500, 1024, 3072), (1500, 768, 2304), (2000, 768, 2304), (5, 1024, 3072)])
+def test_input_gradient_widths_beside_a_weight_gradient(M, N, K):
+    """Input gradients whose tile width depends on what their layer's weight gradient leaves free, on both sides of the line, and
+    that weight gradient. bf16 results: half an ulp, 2^-9 of the value, in the norm; fp32 ones: sums of M terms."""
+    torch.manual_seed(M + N)
+    dy, w, x = (torch.randn(*shape, device="cuda").to(BF) for shape in ((M, K), (K, N), (M, N)))
+    dx = torch.empty(M, N, device="cuda", dtype=BF)
+    assert C.gemm_bf16(dy, w, dx, 2, STORE) == 0
+    assert rel(dx, dy.float() @ w.float()) < 4e-3
+    dw = torch.empty(K, N, device="cuda")
+    assert C.gemm_bf16(dy, x, dw, 1, 4) == 0
+    assert rel(dw, dy.float().t() @ x.float()) < 1e-4
+    assert C.gemm_status()[0] == 0
