@@ -826,21 +826,23 @@ int layernorm_backward(stream_t stream, const void *dy, const void *x, const voi
 
 // --------------------------------------------------------------------------- embedding ----
 namespace {
-// One warp per row: the id is read once, and no element pays for a 64-bit division (one thread per 8 elements of the whole
-// output spent more on that than on its loads). 16384 rows of 768 from fp32 tables: 30 -> 16 us.
+// A warp takes 256 columns of a row at a time, so that the id is read once for them, no element pays for a division, and a piece's
+// loads do not wait for the piece before. One warp for the whole row was slower at both ends: 16384 x 1280 from fp32 tables 26.4 us,
+// 21.3 so; 114 x 1280 5.6 and 3.2 (cold caches).
 __global__ void __launch_bounds__(256) embedding_fwd_kernel(const int64_t *__restrict__ idx, const void *__restrict__ wte,
                                                             const void *__restrict__ wpe, int tdt,
                                                             __nv_bfloat16 *__restrict__ out, int64_t rows,
                                                             int64_t seq_len, int d, int64_t vocab) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
+  const int lane = threadIdx.x & 31, pieces = (d + 255) / 256;
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5), items = rows * pieces;
+  for (int64_t item = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); item < items; item += warps) {
+    const int64_t row = items < INT32_MAX ? static_cast<int32_t>(item) / pieces : item / pieces;
     int64_t token = idx[row];
     (void)CS_IN_BOUNDS(kKidEmbeddingFwd, token, vocab);  // diagnostic build: remember the first bad id
     token = token < 0 ? 0 : (token >= vocab ? vocab - 1 : token);  // clamp instead of faulting
-    const int64_t pos = wpe ? row % seq_len : 0;
-#pragma unroll 4
-    for (int col = lane * 8; col < d; col += 256) {
+    const int64_t pos = !wpe ? 0 : (rows < INT32_MAX && seq_len < INT32_MAX ? static_cast<int32_t>(row) % static_cast<int32_t>(seq_len) : row % seq_len);
+    const int col = static_cast<int>(item - row * pieces) * 256 + lane * 8;
+    if (col < d) {
       float a[8];
       load8(wte, token * d + col, tdt, a);
       if (wpe) {
@@ -854,22 +856,25 @@ __global__ void __launch_bounds__(256) embedding_fwd_kernel(const int64_t *__res
   }
 }
 
-// One warp per row, four columns per atomic: a vector reduction carries four times what a scalar one does through the same
+// One warp per row (several where rows are few), four columns per atomic: a vector reduction carries four times what a scalar one does through the same
 // L2 slot, and text sends a good part of its rows to the same few ids. 16384 rows of 768, ids log-uniform over 50304:
 // 143 -> 24 us. kVector: the table is 16-byte aligned.
-template <bool kVector>
+template <bool kVector, bool kSplit>
 __global__ void __launch_bounds__(256) embedding_bwd_wte_kernel(const int64_t *__restrict__ idx,
                                                                 const __nv_bfloat16 *__restrict__ dy,
                                                                 float *__restrict__ dwte, int64_t rows, int d,
-                                                                int64_t vocab, int64_t padding_idx) {
+                                                                int64_t vocab, int64_t padding_idx, int segments) {
+  const int segs = kSplit ? segments : 1;
   const int lane = threadIdx.x & 31;
   const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
+  for (int64_t item = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); item < rows * segs; item += warps) {
+    const int64_t row = item / segs;
+    const int seg = static_cast<int>(item - row * segs);
     const int64_t token = idx[row];
     if (token != padding_idx) (void)CS_IN_BOUNDS(kKidEmbeddingBwd, token, vocab);
     if (token < 0 || token >= vocab || token == padding_idx) continue;
 #pragma unroll 4
-    for (int col = lane * 4; col < d; col += 128) {
+    for (int col = (seg * 32 + lane) * 4; col < d; col += 128 * segs) {
       const uint2 raw = *reinterpret_cast<const uint2 *>(dy + row * d + col);
       const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
       const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
@@ -913,10 +918,20 @@ int embedding_forward(stream_t stream, const int64_t *idx, const void *wte, cons
                       int64_t rows, int64_t seq_len, int64_t d, int64_t vocab) {
   if (rows == 0) return 0;
   if (d % 8 != 0) return static_cast<int>(cudaErrorInvalidValue);
-  embedding_fwd_kernel<<<grid_for(rows * 32, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  embedding_fwd_kernel<<<grid_for(rows * ((d + 255) / 256) * 32, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       idx, wte, wpe, table_dtype, static_cast<__nv_bfloat16 *>(out), rows, seq_len, static_cast<int>(d), vocab);
   return finish_launch();
 }
+
+namespace {
+// Warps per row: a row is split while that leaves each warp a piece and the SMs have fewer than sixteen warps each. 114 rows of
+// 1280: 4.5 us with one warp each, 2.7 so (cold caches); 4096 rows of 768 gain nothing from it.
+int embedding_segments(int64_t rows, int64_t d, int64_t piece) {
+  int segs = 1;
+  while (segs * piece < d && rows * segs < 16 * kSmCount) segs *= 2;
+  return segs;
+}
+}  // namespace
 
 int embedding_backward(stream_t stream, const int64_t *idx, const void *dy, float *dwte, float *dwpe, int accumulate_wpe,
                        int64_t rows, int64_t seq_len, int64_t d, int64_t vocab, int64_t padding_idx) {
@@ -924,9 +939,12 @@ int embedding_backward(stream_t stream, const int64_t *idx, const void *dy, floa
   if (rows == 0) return 0;
   if (d % 8 != 0) return static_cast<int>(cudaErrorInvalidValue);
   if (dwte) {
-    auto *kernel = (reinterpret_cast<uintptr_t>(dwte) & 15) == 0 ? embedding_bwd_wte_kernel<true> : embedding_bwd_wte_kernel<false>;
-    kernel<<<grid_for(rows * 32, 256), 256, 0, s>>>(idx, static_cast<const __nv_bfloat16 *>(dy), dwte, rows, static_cast<int>(d), vocab,
-                                                    padding_idx);
+    const int segs = embedding_segments(rows, d, 128);
+    const bool aligned = (reinterpret_cast<uintptr_t>(dwte) & 15) == 0;
+    auto *kernel = segs > 1 ? (aligned ? embedding_bwd_wte_kernel<true, true> : embedding_bwd_wte_kernel<false, true>)
+                            : (aligned ? embedding_bwd_wte_kernel<true, false> : embedding_bwd_wte_kernel<false, false>);
+    kernel<<<grid_for(rows * segs * 32, 256), 256, 0, s>>>(idx, static_cast<const __nv_bfloat16 *>(dy), dwte, rows, static_cast<int>(d),
+                                                           vocab, padding_idx, segs);
   }
   if (dwpe)
     embedding_bwd_wpe_kernel<<<grid_for(seq_len * (d / 8), 256), 256, 0, s>>>(static_cast<const __nv_bfloat16 *>(dy), dwpe,

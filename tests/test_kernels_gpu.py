@@ -472,3 +472,25 @@ def test_classifier_loss_over_vocabulary_sizes(gpu_scheduler, rows, vocab, padde
     dw[:vocab] = logits.grad.t() @ x.double()
     assert ((dx.raw().double() - logits.grad @ w[:vocab]).norm() / (logits.grad @ w[:vocab]).norm()).item() < 5e-3
     assert ((lin.grad_weight.raw().double() - dw).norm() / dw.norm()).item() < 5e-3
+
+
+@pytest.mark.parametrize("batch,seq,d", [(1, 1, 8), (2, 57, 1280), (3, 5, 264), (1, 37, 1288), (4, 592, 264), (3, 790, 264), (5, 1000, 768)])
+def test_token_and_position_embedding_pieces(gpu_scheduler, batch, seq, d):
+    """Rows of one piece and several, whole and not, on both sides of the row count from which backward gives a row one warp. The
+    forward sum is one fp32 addition, rounded once; gradients are fp32 sums of at most batch * seq terms."""
+    s = gpu_scheduler
+    torch.manual_seed(batch * seq + d)
+    V = 30
+    te, pe = C.embedding_init(s, V, d), C.embedding_init(s, 1024, d)
+    idx = torch.randint(0, V, (batch, seq), device="cuda")
+    dy = torch.randn(batch, seq, d, device="cuda").to(BF)
+    with cs.autocast(s, BF):
+        y = C.embedding_forward_token_position(s, te, pe, T(idx))
+    C.embedding_backward_token_position(s, te, pe, T(dy))
+    s.synchronize()
+    assert torch.equal(y.raw(), (te.weight.raw()[idx] + pe.weight.raw()[:seq]).to(BF))
+    want = torch.zeros(V, d, device="cuda", dtype=torch.float64).index_add_(0, idx.view(-1), dy.double().view(-1, d))
+    size = torch.zeros(V, d, device="cuda", dtype=torch.float64).index_add_(0, idx.view(-1), dy.double().abs().view(-1, d))
+    count = torch.bincount(idx.view(-1), minlength=V)[:, None]
+    assert ((te.grad_weight.raw().double() - want).abs() <= count * 2.0 ** -24 * size).all()
+    assert ((pe.grad_weight.raw()[:seq].double() - dy.double().sum(0)).abs() <= batch * 2.0 ** -24 * dy.double().abs().sum(0)).all()
