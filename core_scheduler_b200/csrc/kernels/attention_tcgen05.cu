@@ -149,6 +149,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&v)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+               : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(
@@ -210,17 +220,6 @@ __device__ __forceinline__ void mask_columns(uint32_t (&v)[32], uint32_t keep) {
 #pragma unroll
   for (int i = 0; i < 32; ++i)
     if (!((keep >> i) & 1u)) v[i] = 0xff800000u;
-}
-
-// Masked elements of a row of P' or dS' (two bf16 a word) become zero. After the exponential: a score masked before it is undone by a
-// log-sum-exp that is not finite or a scale that is not positive, and a NaN of one query would reach the keys it cannot see.
-// Only tiles on the diagonal pay for it: 16 x 1024 tokens, 12 heads, all of backward 148 us with the mask before, 147 with it here.
-__device__ __forceinline__ void mask_pairs(uint32_t (&v)[16], uint32_t keep) {
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    if (!((keep >> (2 * i)) & 1u)) v[i] &= 0xffff0000u;
-    if (!((keep >> (2 * i + 1)) & 1u)) v[i] &= 0x0000ffffu;
-  }
 }
 
 struct AttnParams {
@@ -519,15 +518,22 @@ struct AttnBwdParams {
   const float *neg_lse;    // [B, H, T]: -lse * log2(e)
   const float *neg_delta;  // [B, H, T]: -delta
   int B, T, H;
-  float scale, scale_log2e;
+  float scale;             // factor of dQ and dK
+  float scale_log2e;       // magnitude of the scale (never zero) * log2(e)
   DeviceStatus *status;
   int causal;
+  int negate;              // as in the forward pass
 };
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
                "r"(bytes), "r"(bar)
                : "memory");
+}
+__device__ __forceinline__ float ld_shared(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
 }
 __device__ __forceinline__ void ld_shared_pairs(uint32_t addr, F2 &a, F2 &b) {
   asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a.v), "=l"(b.v) : "r"(addr));
@@ -592,10 +598,69 @@ __device__ __forceinline__ BwdItem bwd_item(const AttnBwdParams &p, int id) {
 // the longest one of every round.
 __device__ __forceinline__ int bwd_deal(int k) { return k * gridDim.x + ((k & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x); }
 
+// barriers that the softmax groups use
+constexpr int BWD_SDP_FULL = 6, BWD_PDS_FULL = BWD_SDP_FULL + BWD_GROUPS, BWD_C_FULL = BWD_PDS_FULL + 2 * BWD_GROUPS;
+
+// What a softmax group of dK/dV does under a causal mask in a CTA with a query whose log-sum-exp is not finite. -inf for a masked
+// score does not survive that, and the query's NaN would reach the keys it cannot see: here masked elements are cleared after the
+// exponential. A function of its own, eight columns at a time: in the loop that every other CTA runs, the second mask cost
+// registers and spills (dK/dV of 2 x 4096 tokens, 20 heads: 157 us without it, 166 with it there, 161 so).
+__device__ __noinline__ void careful_dkdv(const AttnBwdParams &p, uint32_t s_tmem, uint32_t vec_smem, uint32_t bar_base,
+                                          volatile int *abort_flag, int g, int r, int items) {
+  const uint32_t dp_tmem = s_tmem + BC;
+  const int lane = r & 31;
+  int next = g, s = g;
+  uint32_t cph = 0, parity = 0;
+  for (int k = 0, id; (id = bwd_deal(k)) < items; ++k) {
+    const int n_iter = bwd_item<true>(p, id).n_iter;
+    for (; next < n_iter; next += BWD_GROUPS) {
+      if (!mbar_wait_warp(bar_base + 8u * (BWD_C_FULL + s), cph, abort_flag)) return;
+      if (!mbar_wait_warp(bar_base + 8u * (BWD_SDP_FULL + g), parity, abort_flag)) return;
+      parity ^= 1u;
+      fence_after();
+      const uint32_t vec = vec_smem + s * 512;
+#pragma unroll 1
+      for (int c = 0; c < BC; c += 8) {
+        uint32_t sv[8], dv[8], pp[4], dd[4];
+        tmem_ld8(s_tmem + c, sv);
+        tmem_ld8(dp_tmem + c, dv);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+          float pr[2], ds[2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const uint32_t at = vec + (c + i + j) * 4;
+            const bool seen = next * BC + c + i + j >= r;  // tiles start at the block's own rows
+            pr[j] = seen ? fast_exp2(fmaf(__uint_as_float(sv[i + j]), p.scale_log2e, ld_shared(at))) : 0.f;
+            ds[j] = seen ? pr[j] * (__uint_as_float(dv[i + j]) + ld_shared(at + 256)) : 0.f;
+          }
+          pp[i >> 1] = pack2(pr[0], pr[1]);
+          dd[i >> 1] = pack2(ds[0], ds[1]);
+        }
+        // over the scores of columns up to c / 2 + 3, which this warp has read
+        tmem_st4(s_tmem + c / 2, pp);
+        tmem_st4(dp_tmem + c / 2, dd);
+      }
+      tmem_wait_st();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_base + 8u * (BWD_PDS_FULL + g));
+      s += BWD_GROUPS;
+      if (s >= BWD_STAGES) {
+        s -= BWD_STAGES;
+        cph ^= 1u;
+      }
+    }
+    next -= n_iter;
+  }
+}
+
 template <bool kDKV>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_constant__ CUtensorMap qkv_c,
-                     const __grid_constant__ CUtensorMap do_r, const __grid_constant__ CUtensorMap do_c, const AttnBwdParams p) {
+                     const __grid_constant__ CUtensorMap do_r, const __grid_constant__ CUtensorMap do_c,
+                     const __grid_constant__ AttnBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *aligned = smem_raw + (base - smem_u32(smem_raw));
@@ -605,8 +670,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
   const uint32_t vec_smem = c_smem + STAGES * 2 * C_TILE_BYTES;  // per stage: -lse[64], -delta[64] of the streamed queries
   const uint32_t bar_base = vec_smem + STAGES * 512;
   uint64_t *bars = reinterpret_cast<uint64_t *>(aligned + (bar_base - base));
-  enum { R_FULL = 0, R_EMPTY = 2, ACC_FULL = 4, ACC_EMPTY, SDP_FULL, PDS_FULL = SDP_FULL + GROUPS, PDS_EMPTY = PDS_FULL + GROUPS,
-         C_FULL = PDS_EMPTY + GROUPS,
+  enum { R_FULL = 0, R_EMPTY = 2, ACC_FULL = 4, ACC_EMPTY, SDP_FULL = BWD_SDP_FULL, PDS_FULL = BWD_PDS_FULL, PDS_EMPTY = PDS_FULL + GROUPS,
+         C_FULL = BWD_C_FULL,
          C_EMPTY = C_FULL + STAGES, NUM_BARS = C_EMPTY + STAGES };
   auto bar = [&](int i) { return bar_base + 8u * i; };
   volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(bars + NUM_BARS);
@@ -693,6 +758,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
   } else if (warp == 1) {
     // S' and dP' of every tile, as soon as its buffer is free: M=128, N=64, both operands K-major
     constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BC >> 3) << 17) | (8u << 24);
+    const uint32_t idesc_s = idesc | (p.negate ? 1u << 13 : 0u);
     // descriptors are built once; a k-step, a stage or a buffer only advances the 16-byte-unit address field
     const uint64_t d_r1 = smem_desc(r_smem, 16, 1024), d_r2 = smem_desc(r_smem + TILE_BYTES, 16, 1024);
     const uint64_t d_c1 = smem_desc(c_smem, 16, 1024), d_c2 = smem_desc(c_smem + C_TILE_BYTES, 16, 1024);
@@ -713,7 +779,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
         const uint32_t s_tmem = tmem_base + g * 2 * BC;
         if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk) umma(s_tmem, d_r1 + rt + kk * kStepK, d_c1 + at + kk * kStepK, idesc, kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < HD / 16; ++kk) umma(s_tmem, d_r1 + rt + kk * kStepK, d_c1 + at + kk * kStepK, idesc_s, kk > 0 ? 1u : 0u);
 #pragma unroll
           for (int kk = 0; kk < HD / 16; ++kk) umma(s_tmem + BC, d_r2 + rt + kk * kStepK, d_c2 + at + kk * kStepK, idesc, kk > 0 ? 1u : 0u);
           umma_commit(bar(SDP_FULL + g));
@@ -773,87 +839,107 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap qkv_r, const __grid_con
     const int g = (warp - 4) >> 2;   // softmax group: tiles g, g + GROUPS, ...
     const int r = q * 32 + lane;     // row of the resident block
     const uint32_t s_tmem = tmem_base + g * 2 * BC + (static_cast<uint32_t>(q * 32) << 16), dp_tmem = s_tmem + BC;
-    const F2 scale2 = f2(p.scale_log2e, p.scale_log2e);
-    int next = g;        // steps until this group's next tile, counted from the start of a block
-    int s = g;           // stage of that tile
-    uint32_t cph = 0, parity = 0;
-    bool ok = true;
-    for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
-      const BwdItem it = bwd_item<kDKV>(p, id);
-      if (next >= it.n_iter) {
-        next -= it.n_iter;
-        continue;
+    // Does any query on the diagonal of this CTA's blocks have a log-sum-exp that is not finite? Asked while the first tiles are on
+    // their way, by every warp for itself.
+    bool finite = true;
+    if (kDKV && p.causal) {
+      for (int k0 = 0; bwd_deal(k0) < items; k0 += 4) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {  // all loads of a step in flight; past the last block the step's first once more
+          const int id = bwd_deal(k0 + u);
+          const BwdItem it = bwd_item<kDKV>(p, id < items ? id : bwd_deal(k0));
+          v[u] = __ldg(reinterpret_cast<const float4 *>(p.neg_lse + (static_cast<long long>(it.b) * p.H + it.h) * p.T + it.r0) + lane);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)  // 0 * x is zero for finite x only
+          finite &= (0.f * v[u].x + 0.f * v[u].y) + (0.f * v[u].z + 0.f * v[u].w) == 0.f;
       }
-      float lse_r = 0.f, delta_r = 0.f;
-      if (!kDKV) {
-        const long long at = (static_cast<long long>(it.b) * p.H + it.h) * p.T + it.r0 + r;
-        lse_r = p.neg_lse[at];
-        delta_r = p.neg_delta[at];
-      }
-      const F2 lse_r2 = f2(lse_r, lse_r), delta_r2 = f2(delta_r, delta_r);
-      for (; next < it.n_iter; next += GROUPS) {
-        if (kDKV) {
-          ok = mbar_wait_warp(bar(C_FULL + s), cph, abort_flag);  // -lse / -delta of the streamed queries
+      finite = __all_sync(0xffffffffu, finite);
+    }
+    if (kDKV && !finite) {
+      careful_dkdv(p, s_tmem, vec_smem, bar_base, abort_flag, g, r, items);
+    } else {
+      const F2 scale2 = f2(p.scale_log2e, p.scale_log2e);
+      int next = g;        // steps until this group's next tile, counted from the start of a block
+      int s = g;           // stage of that tile
+      uint32_t cph = 0, parity = 0;
+      bool ok = true;
+      for (int k = 0, id; ok && (id = bwd_deal(k)) < items; ++k) {
+        const BwdItem it = bwd_item<kDKV>(p, id);
+        if (next >= it.n_iter) {
+          next -= it.n_iter;
+          continue;
+        }
+        float lse_r = 0.f, delta_r = 0.f;
+        if (!kDKV) {
+          const long long at = (static_cast<long long>(it.b) * p.H + it.h) * p.T + it.r0 + r;
+          lse_r = p.neg_lse[at];
+          delta_r = p.neg_delta[at];
+        }
+        const F2 lse_r2 = f2(lse_r, lse_r), delta_r2 = f2(delta_r, delta_r);
+        for (; next < it.n_iter; next += GROUPS) {
+          if (kDKV) {
+            ok = mbar_wait_warp(bar(C_FULL + s), cph, abort_flag);  // -lse / -delta of the streamed queries
+            if (!ok) break;
+          }
+          ok = mbar_wait_warp(bar(SDP_FULL + g), parity, abort_flag);
           if (!ok) break;
-        }
-        ok = mbar_wait_warp(bar(SDP_FULL + g), parity, abort_flag);
-        if (!ok) break;
-        parity ^= 1u;
-        fence_after();
-        // Rows are keys and columns queries (kDKV), or rows queries and columns keys; keep key <= query. `edge` is the column
-        // of this row's own position: dK/dV masks the columns before it, dQ those after it.
-        const int c0 = (it.c_first + next) * BC - it.r0;  // first streamed row, relative to the resident block
-        const int edge = p.causal ? r - c0 : (kDKV ? -1 : BC);
-        const uint32_t vec = vec_smem + s * 512;
+          parity ^= 1u;
+          fence_after();
+          const int c0 = (it.c_first + next) * BC - it.r0;  // first streamed row, relative to the resident block
+          // rows are keys and columns queries (kDKV), or rows queries and columns keys: keep key <= query
+          const bool masked = p.causal && (kDKV ? c0 < 128 : c0 + BC > 0);
+          const uint32_t vec = vec_smem + s * 512;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {  // 32 columns at a time
-          uint32_t sv[32], dv[32];
-          tmem_ld32(s_tmem + c * 32, sv);
-          tmem_ld32(dp_tmem + c * 32, dv);
-          tmem_wait_ld();
-          uint32_t pp[16], dd[16];
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            F2 nl[2] = {lse_r2, lse_r2}, nd[2] = {delta_r2, delta_r2};
-            if (kDKV) {
-              ld_shared_pairs(vec + (c * 32 + i) * 4, nl[0], nl[1]);
-              ld_shared_pairs(vec + 256 + (c * 32 + i) * 4, nd[0], nd[1]);
+          for (int c = 0; c < 2; ++c) {  // 32 columns at a time
+            uint32_t sv[32], dv[32];
+            tmem_ld32(s_tmem + c * 32, sv);
+            tmem_ld32(dp_tmem + c * 32, dv);
+            tmem_wait_ld();
+            if (masked) {
+              const int first = r - c0 - c * 32;  // dK/dV: columns below it are masked; dQ: columns above it
+              mask_columns(sv, kDKV ? columns_from(first) : ~columns_from(first + 1));
             }
+            uint32_t pp[16], dd[16];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const int e = i + 2 * j;
-              float a, d;
-              f2_split(f2_fma(f2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), scale2, nl[j]), a, d);
-              const F2 pr = f2(fast_exp2(a), fast_exp2(d));
-              const F2 ds = f2_mul(pr, f2_add(f2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), nd[j]));
+            for (int i = 0; i < 32; i += 4) {
+              F2 nl[2] = {lse_r2, lse_r2}, nd[2] = {delta_r2, delta_r2};
               if (kDKV) {
-                f2_split(pr, a, d);
-                pp[e >> 1] = pack2(a, d);
+                ld_shared_pairs(vec + (c * 32 + i) * 4, nl[0], nl[1]);
+                ld_shared_pairs(vec + 256 + (c * 32 + i) * 4, nd[0], nd[1]);
               }
-              f2_split(ds, a, d);
-              dd[e >> 1] = pack2(a, d);
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                const int e = i + 2 * j;
+                float a, d;
+                f2_split(f2_fma(f2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), scale2, nl[j]), a, d);
+                const F2 pr = f2(fast_exp2(a), fast_exp2(d));
+                const F2 ds = f2_mul(pr, f2_add(f2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), nd[j]));
+                if (kDKV) {
+                  f2_split(pr, a, d);
+                  pp[e >> 1] = pack2(a, d);
+                }
+                f2_split(ds, a, d);
+                dd[e >> 1] = pack2(a, d);
+              }
             }
+            // over the scores of columns 0..31, which this warp has read
+            if (kDKV) tmem_st16(s_tmem + c * 16, pp);
+            tmem_st16(dp_tmem + c * 16, dd);
           }
-          if (__any_sync(0xffffffffu, kDKV ? edge > c * 32 : edge < c * 32 + 31)) {
-            const uint32_t keep = kDKV ? columns_from(edge - c * 32) : ~columns_from(edge + 1 - c * 32);
-            if (kDKV) mask_pairs(pp, keep);
-            mask_pairs(dd, keep);
+          tmem_wait_st();
+          fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(PDS_FULL + g));
+          s += GROUPS;
+          if (s >= STAGES) {
+            s -= STAGES;
+            cph ^= 1u;
           }
-          // over the scores of columns 0..31, which this warp has read
-          if (kDKV) tmem_st16(s_tmem + c * 16, pp);
-          tmem_st16(dp_tmem + c * 16, dd);
         }
-        tmem_wait_st();
-        fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(PDS_FULL + g));
-        s += GROUPS;
-        if (s >= STAGES) {
-          s -= STAGES;
-          cph ^= 1u;
-        }
+        next -= it.n_iter;
       }
-      next -= it.n_iter;
     }
   } else if (warp >= 4 + 4 * GROUPS) {
     // accumulators -> dqkv: thread = row; dV and dK, or dQ
@@ -934,6 +1020,15 @@ DeviceStatus *attn_status_ptr() {
 }
 }  // namespace
 
+namespace {
+// The running maximum, -inf for masked scores and the lag of the reference want a positive scale: a negative one is its magnitude
+// with the products negated, and zero the smallest normal number, which leaves every finite score at exp(0).
+float scale_magnitude(float scale) {
+  const float magnitude = std::fabs(scale);
+  return magnitude < FLT_MIN ? FLT_MIN : magnitude;
+}
+}  // namespace
+
 int attention_forward_packed(stream_t stream, const void *qkv, void *out, float *lse, int64_t B, int64_t T, int64_t H, int64_t D,
                              float scale, int causal) {
   if (D != HD || T % BQ != 0 || B <= 0 || H <= 0 || T <= 0) return -1;
@@ -951,11 +1046,8 @@ int attention_forward_packed(stream_t stream, const void *qkv, void *out, float 
   p.B = static_cast<int>(B);
   p.T = static_cast<int>(T);
   p.H = static_cast<int>(H);
-  // The kernel's maximum, its -inf for masked keys and the lag of its reference want a positive scale: a negative one is its
-  // magnitude with the products negated, and zero the smallest normal number, which leaves every finite score at exp(0).
-  const float magnitude = std::fabs(scale);
   p.negate = scale < 0.f ? 1 : 0;
-  p.scale = magnitude < FLT_MIN ? FLT_MIN : magnitude;
+  p.scale = scale_magnitude(scale);
   p.scale_log2e = p.scale * 1.4426950408889634f;
   p.status = attn_status_ptr();
   p.causal = causal ? 1 : 0;
@@ -992,7 +1084,8 @@ int attention_backward_packed(stream_t stream, const void *qkv, const void *out,
   p.T = static_cast<int>(T);
   p.H = static_cast<int>(H);
   p.scale = scale;
-  p.scale_log2e = scale * 1.4426950408889634f;
+  p.scale_log2e = scale_magnitude(scale) * 1.4426950408889634f;
+  p.negate = scale < 0.f ? 1 : 0;
   p.status = attn_status_ptr();
   p.causal = causal ? 1 : 0;
   const int64_t items = T / 128 * H * B;
