@@ -828,7 +828,8 @@ int layernorm_backward(stream_t stream, const void *dy, const void *x, const voi
 namespace {
 // A warp takes 256 columns of a row at a time, so that the id is read once for them, no element pays for a division, and a piece's
 // loads do not wait for the piece before. One warp for the whole row was slower at both ends: 16384 x 1280 from fp32 tables 26.4 us,
-// 21.3 so; 114 x 1280 5.6 and 3.2 (cold caches).
+// 21.3 so; 114 x 1280 5.6 and 3.2 (cold caches). Four CTAs an SM leave room for what runs beside it: embed forward + backward of
+// 16384 x 768, one pass after another, 69 us with eight and 64 with four.
 __global__ void __launch_bounds__(256) embedding_fwd_kernel(const int64_t *__restrict__ idx, const void *__restrict__ wte,
                                                             const void *__restrict__ wpe, int tdt,
                                                             __nv_bfloat16 *__restrict__ out, int64_t rows,
@@ -918,7 +919,7 @@ int embedding_forward(stream_t stream, const int64_t *idx, const void *wte, cons
                       int64_t rows, int64_t seq_len, int64_t d, int64_t vocab) {
   if (rows == 0) return 0;
   if (d % 8 != 0) return static_cast<int>(cudaErrorInvalidValue);
-  embedding_fwd_kernel<<<grid_for(rows * ((d + 255) / 256) * 32, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  embedding_fwd_kernel<<<grid_for(rows * ((d + 255) / 256) * 32, 256, 4), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       idx, wte, wpe, table_dtype, static_cast<__nv_bfloat16 *>(out), rows, seq_len, static_cast<int>(d), vocab);
   return finish_launch();
 }
