@@ -10,7 +10,7 @@
 //              running sum, exponentiates on packed pairs and writes P back to TMEM. O accumulates in TMEM across key
 //              blocks; a warp rescales its 32 rows of O in place only when a row maximum has grown by more than 2^8 since
 //              the reference was taken (probabilities stay below 256, exact after the final division)
-// Two CTAs share an SM (81 KB of shared memory, 256 TMEM columns, 168 registers a thread): one's barriers and loads hide
+// Two CTAs share an SM (81 KB of shared memory, 256 TMEM columns, 154 registers a thread): one's barriers and loads hide
 // behind the other's exponentials, 1024 cycles a block and what bounds it. 16 x 1024 tokens, 12 heads, causal: 102 -> 58 us
 // against four CTAs with 64-key blocks that read S twice and passed P through shared memory; 2 x 4096, 20 heads
 // 289 -> 122. Scores never touch global memory. Every mbarrier wait is bounded (abort flag + status word).
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS_PER_SM) attention_fwd_kernel
 // tile, the score buffer of the next one ready, ran in step with each other and needed 2250 cycles for 128 columns, two CTAs
 // an SM with 64-column tiles 2800. The accumulators are drained by four warps of their own while the next block is under
 // way, across whose boundary the pipeline runs on; resident tiles are double-buffered. 16 x 1024 tokens, 12 heads, causal:
-// dK/dV 138 -> 78 us, dQ 91 -> 59; 2 x 4096, 20 heads 343 -> 164 and 231 -> 135.
+// dK/dV 138 -> 78 us, dQ 91 -> 53; 2 x 4096, 20 heads 343 -> 161 and 231 -> 127.
 constexpr int BC = 64;                          // streamed rows per step
 constexpr int C_TILE_BYTES = BC * HD * 2;       // 8 KB
 constexpr int BWD_GROUPS = 3;                   // softmax groups and score buffers
